@@ -213,7 +213,9 @@ def run_ours(args, world, rank, local):
     wall = time.perf_counter() - t_wall
     launches = ctx.launch_count() - launches0
     clk = clocks.stop() if rank == 0 else None
+    before = ctx.field_applied()
     st = ctx.stats(sptr)
+    st["applied"] = ctx.field_applied() - before
     ms = max_over_ranks(world, statistics.mean(step_ms))
     value = world * n / (ms * 1e-3) / 1e9
 
@@ -261,7 +263,7 @@ def run_ours(args, world, rank, local):
     # roofline of the FP32 bulk kernel (FMA-pipe bound)
     peak = lib.fma_probe(local)
     bulk = statistics.mean(bulk_ms)
-    flops = field_flops(rs, st["voxel_iters"])
+    flops = field_flops(rs, st["applied"])  # what the kernel carried out
     achieved = flops / (bulk * 1e-3) / 1e12
 
     # end to end through the host-buffer entry point, pinned host output
@@ -336,7 +338,7 @@ def run_ours(args, world, rank, local):
         "field_stats": dict(st, bulk_ms=bulk, refine_ms=statistics.mean(refine_ms),
                             wall_s=wall, refined_frac=st["refined"] / n,
                             gvoxel_iterations_s=world * st["voxel_iters"] / (ms * 1e-3) / 1e9,
-                            lane_efficiency=st["voxel_iters"] / max(1, st["lane_iters"])),
+                            lane_efficiency=st["applied"] / max(1, st["lane_iters"])),
         "roofline": {"bound": "fma", "kernel": "field32x2_kernel", "achieved": achieved,
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": TRAFFIC_PER_VOXEL * n,

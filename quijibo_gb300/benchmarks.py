@@ -61,9 +61,11 @@ def bench_mesh(args):
         raise SystemExit("raise --vert-cap/--tri-cap: needs %d / %d" % (st["n_verts"], st["n_tris"]))
     torch.cuda.synchronize()
     t0 = time.perf_counter()
+    before = ctx.field_applied()
     _, st = ctx.mesh_stream(h, g, it, **kw)
     torch.cuda.synchronize()
     wall = time.perf_counter() - t0
+    applied = ctx.field_applied() - before
     # the field alone over the same grid, for the split
     f = torch.empty(g.res[0] * g.res[1] * min(g.res[2], args.slab + 1), dtype=torch.float64,
                     device="cuda")
@@ -83,7 +85,7 @@ def bench_mesh(args):
             "bisection_map_evals_ff": st["map_evals_ff"], "unbracketed": st["n_unbracketed"],
             "degenerate": st["n_degenerate"], "slabs": st["slabs"],
             "refined": st["field"]["refined"],
-            "lane_efficiency": st["field"]["voxel_iters"] / max(1, st["field"]["lane_iters"])}
+            "lane_efficiency": applied / max(1, st["field"]["lane_iters"])}
 
 
 def bench_classify(args):
@@ -618,8 +620,10 @@ def bench_large(args):
         e0, e1 = _events(torch)
         t0 = time.perf_counter()
         e0.record()
+        before = ctx.field_applied()
         rc, st = ctx.mesh_stream(h, g, it, check=False, d_verts32=v32.data_ptr(), vert_cap=vcap,
                                  d_tris=tris.data_ptr(), tri_cap=tcap, slab_nz=args.slab)
+        applied = ctx.field_applied() - before
         e1.record()
         torch.cuda.synchronize()
         wall = time.perf_counter() - t0
@@ -629,7 +633,7 @@ def bench_large(args):
         mesh_ms = st["ms_classify"] + st["ms_triangles"]
         alg = mesh_algorithmic_bytes(n, V, T)
         fs = st["field"]
-        flops = field_flops(rs, fs["voxel_iters"])
+        flops = field_flops(rs, applied)
         bulk = st["ms_field_bulk"]
         field_gvox = n / (st["ms_field"] * 1e-3) / 1e9
         out["mesh"] = {"passes": 1, "triangles": st["n_tris"], "vertices": V,
@@ -654,7 +658,7 @@ def bench_large(args):
                                      "achieved_tflops": flops / (bulk * 1e-3) / 1e12,
                                      "peak_tflops": peak,
                                      "frac": flops / (bulk * 1e-3) / 1e12 / peak},
-                        "lane_efficiency": fs["voxel_iters"] / max(1, fs["lane_iters"])}
+                        "lane_efficiency": applied / max(1, fs["lane_iters"])}
         del v32, tris
         torch.cuda.empty_cache()
 
@@ -664,6 +668,7 @@ def bench_large(args):
         buf = torch.empty(args.slab * XY, dtype=torch.float64, device="cuda")
         bulk = rest = 0.0
         tot = {}
+        before = ctx.field_applied()
         for z0 in range(0, g.res[2], args.slab):
             z1 = min(z0 + args.slab, g.res[2])
             ctx.field(h, g, it, buf.data_ptr(), z0=z0, z1=z1)
@@ -672,14 +677,15 @@ def bench_large(args):
             for k, v in ctx.stats().items():
                 tot[k] = tot.get(k, 0) + v
         del buf
-        flops = field_flops(rs, tot["voxel_iters"])
+        applied = ctx.field_applied() - before
+        flops = field_flops(rs, applied)
         field_gvox = n / ((bulk + rest) * 1e-3) / 1e9
         out["field_alone"] = {
             "gvox_s": field_gvox, "bulk_ms": bulk, "rest_ms": rest,
             "gvoxel_iterations_s": tot["voxel_iters"] / ((bulk + rest) * 1e-3) / 1e9,
             "roofline": {"achieved_tflops": flops / (bulk * 1e-3) / 1e12, "peak_tflops": peak,
                          "frac": flops / (bulk * 1e-3) / 1e12 / peak},
-            "stats": tot, "lane_efficiency": tot["voxel_iters"] / max(1, tot["lane_iters"])}
+            "stats": tot, "lane_efficiency": applied / max(1, tot["lane_iters"])}
 
     # (3) sampled slices: precision form against both FP64 forms
     if args.check_slices > 0:

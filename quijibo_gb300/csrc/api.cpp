@@ -372,6 +372,7 @@ int qjg_field_stats_read(qjg_ctx* ctx, void* stream, qjg_field_stats* out) {
   out->lane_iters = (int64_t)st.aux[3];
   out->rerun = (int64_t)st.rerun;
   out->rerun_iters = (int64_t)st.rerun_iters;
+  ctx->applied += (int64_t)st.applied;
   return QJG_OK;
 }
 
@@ -453,6 +454,7 @@ int qjg_field_host(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg
     total.lane_iters += (int64_t)st.aux[3];
     total.rerun += (int64_t)st.rerun;
     total.rerun_iters += (int64_t)st.rerun_iters;
+    ctx->applied += (int64_t)st.applied;
   }
   if (stats) *stats = total;
   return QJG_OK;
@@ -478,6 +480,8 @@ int qjg_last_timings(qjg_ctx* ctx, float* ms_bulk, float* ms_refine) {
   if (ctx->timed_refine) QJ_CUDA(ctx, cudaEventElapsedTime(ms_refine, ctx->ev[1], ctx->ev[2]));
   return QJG_OK;
 }
+
+int64_t qjg_field_applied(qjg_ctx* ctx) { return ctx ? ctx->applied : -1; }
 
 int64_t qjg_launch_count(qjg_ctx* ctx) { return ctx ? ctx->launches : -1; }
 

@@ -1375,6 +1375,7 @@ __global__ void mc_stats_add_kernel(DevStats* acc, const DevStats* st) {
   for (int k = 0; k < 4; k++) acc->aux[k] += st->aux[k];
   acc->rerun += st->rerun;
   acc->rerun_iters += st->rerun_iters;
+  acc->applied += st->applied;
   acc->ff_evals += st->ff_evals;
 }
 

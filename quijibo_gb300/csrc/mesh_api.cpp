@@ -615,6 +615,7 @@ int qjg_mesh_async_result(qjg_ctx* ctx, qjg_mesh_stats* stats) {
   st.field.lane_iters = (int64_t)fs.aux[3];
   st.field.rerun = (int64_t)fs.rerun;
   st.field.rerun_iters = (int64_t)fs.rerun_iters;
+  ctx->applied += (int64_t)fs.applied;
   *stats = st;
   if (run.overflow)
     return fail(ctx, QJG_ERR_CAPACITY, "the mesh outgrew the capacities of the fixed sequence");

@@ -90,6 +90,8 @@ struct DevStats {
   unsigned long long aux[4];
   unsigned long long rerun;         // length of the double-float re-run list
   unsigned long long rerun_iters;   // map applications of the re-runs
+  unsigned long long applied;       // map applications the FP32 bulk pass carried out (voxel_iters
+                                    // counts orbit lengths, repeating orbits' tails among them)
   unsigned long long ff_evals;      // mesher: double-float evaluations that decided a point
 };
 

@@ -277,6 +277,7 @@ EXPORTS = {
     "qjg_set_timing": ([C.c_void_p, C.c_int], C.c_int),
     "qjg_last_timings": ([C.c_void_p, _fp, _fp], C.c_int),
     "qjg_launch_count": ([C.c_void_p], C.c_int64),
+    "qjg_field_applied": ([C.c_void_p], C.c_int64),
     "qjg_fma_probe": ([C.c_int, _dp], C.c_int),
     "qjg_crmath_eval": ([C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p], C.c_int),
     "qjg_set_field32_pairs": ([C.c_int], C.c_int),
@@ -652,6 +653,10 @@ class Context:
         a, b = C.c_float(), C.c_float()
         self._check(self.L.qjg_last_timings(self.h, C.byref(a), C.byref(b)), "qjg_last_timings")
         return a.value, b.value
+
+    def field_applied(self):
+        """Map applications the FP32 bulk passes carried out so far."""
+        return int(self.L.qjg_field_applied(self.h))
 
     def launch_count(self):
         return int(self.L.qjg_launch_count(self.h))

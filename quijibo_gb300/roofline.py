@@ -3,7 +3,8 @@ bench.py and quijibo_gb300.benchmarks."""
 
 
 def field_flops(rs, voxel_iters, de=True):
-    """Algorithmic FP32 flops of `voxel_iters` map applications (FMA = 2).
+    """Algorithmic FP32 flops of `voxel_iters` map applications (FMA = 2):
+    the ones carried out (Context.field_applied), not the orbit lengths.
 
     Per root term: 4 (q - r) + 11 per squaring (exponent 2) + 28 per
     accumulating Hamilton product (the first root of each product has none)
