@@ -85,8 +85,10 @@ __global__ void __launch_bounds__(128) field64_kernel(const __grid_constant__ Ma
   warp_add(&st->voxel_iters, iters_acc);
 }
 
-// FP64 recomputation of the voxels in `list` (local linear indices).
-template <int POW_REF>
+// FP64 recomputation of the voxels in `list` (local linear indices); the
+// distance estimate (26 of 50 FP64 instructions of a root term with exponent
+// 1) only where the caller wants it.
+template <int POW_REF, bool DE>
 __global__ void __launch_bounds__(128) refine64_kernel(const __grid_constant__ MapParams m,
                                                        const GridParams g,
                                                        const IterParams it, const uint32_t* list,
@@ -111,9 +113,9 @@ __global__ void __launch_bounds__(128) refine64_kernel(const __grid_constant__ M
     cell_center(g, x, y, g.z0 + zl, p);
     int n;
     double d = 0.0;
-    const double f = escape64<POW_REF, true>(m, it, p, g.slice, &n, &d);
+    const double f = escape64<POW_REF, DE>(m, it, p, g.slice, &n, &d);
     field[i] = f;
-    if (de) de[i] = (float)d;
+    if (DE) de[i] = (float)d;
     iters_acc += n;
   }
   warp_add(&st->aux[0], iters_acc);
@@ -301,12 +303,6 @@ struct BulkAcc {
 // 91.5 -> 44.3 ms; 2200 x 2200 x 4, 48 / 24 roots, 60 iterations 83.3 -> 21.8
 // ms; 203 x 171 x 139, 23 / 11 roots, 30 iterations with the distance
 // estimate 9.7 -> 5.2 ms.
-constexpr int ORBIT_WINDOW = 6;  // longest period found
-
-// Steps from one marked iterate to the next: short while orbits of period 1
-// and 2 settle, then long enough for every period up to the window.
-__device__ __forceinline__ int mark_gap(int step) { return step < 12 ? 2 : ORBIT_WINDOW; }
-
 // A thread's marked iterates and the steps since, in shared memory (a
 // register copy would cost the unrolled kernels a resident block).
 struct OrbitLog {
@@ -692,7 +688,8 @@ __global__ void __launch_bounds__(128) refine64_batch_kernel(const BatchTable* _
     cell_center(g, x, y, g.z0 + zl, p);
     int n;
     double d = 0.0;
-    const double f = escape64<false, true>(maps[k], b.it, p, g.slice, &n, &d);
+    const double f = b.de ? escape64<0, true>(maps[k], b.it, p, g.slice, &n, &d)
+                          : escape64<0, false>(maps[k], b.it, p, g.slice, &n, &d);
     b.field[i] = f;
     if (b.de) b.de[i] = (float)d;
     iters_acc += n;
@@ -875,8 +872,12 @@ cudaError_t launch_refine64(const MapParams& m, const GridParams& g, const IterP
   }
 #define QJ_R64(P)                                                                    \
   do {                                                                               \
-    const int blocks = grid_blocks((const void*)refine64_kernel<P>, 128);            \
-    refine64_kernel<P><<<blocks, 128, 0, s>>>(m, g, it, list, st, field, de, st);    \
+    const int blocks = grid_blocks(de ? (const void*)refine64_kernel<P, true>        \
+                                      : (const void*)refine64_kernel<P, false>, 128); \
+    if (de)                                                                          \
+      refine64_kernel<P, true><<<blocks, 128, 0, s>>>(m, g, it, list, st, field, de, st); \
+    else                                                                             \
+      refine64_kernel<P, false><<<blocks, 128, 0, s>>>(m, g, it, list, st, field, de, st); \
   } while (0)
   if (pow_mode == 2)
     QJ_R64(2);
