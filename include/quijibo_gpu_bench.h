@@ -63,8 +63,8 @@ int qjg_set_energy_adjoint_roots(int on);
 int qjg_set_energy_fast(int on);
 
 /* Process-wide block count of the energy forward kernel, for sweeps: 0 (the
- * default) the sizing rule (at least 3 blocks of 128 lanes per SM, more when
- * each lane would otherwise take more than about four samples), else that
+ * default) the sizing rule (the resident blocks in FP32, about four samples a lane
+ * in FP64, at least 3 blocks of 128 lanes per SM), else that
  * many blocks per SM, capped by residency.  With the one-sample kernel (the
  * default) results do not depend on it (each sample's value is its own; sums
  * run in sample order).  Set it while no energy call is in flight; a
@@ -72,7 +72,8 @@ int qjg_set_energy_fast(int on);
 int qjg_set_energy_forward_blocks(int per_sm);
 
 /* Work of the last qjg_energy_forward/backward call on ctx: the map
- * applications of its forward pass (orbit steps of every sample) and the
+ * applications its forward pass carried out (settled orbits are cut short,
+ * so fewer than the orbit steps) and the
  * orbit steps its adjoint ran back over (gradient samples only; 0 for a
  * forward call): the units of the energy kernels' algorithmic FLOP counts. */
 int qjg_energy_last_work(qjg_ctx* ctx, int64_t* applications, int64_t* steps);

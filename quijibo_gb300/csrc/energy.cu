@@ -1053,7 +1053,62 @@ struct SqFwdOut {
   V4<T>* seed_q;    // dE/dq_N per sample (gradient pass)
   T* seed_L;        // dE/dL (constant along the orbit)
   V4<T>* ck;        // q_n at n = 0, SQ_CK, 2 SQ_CK, ...: ck[(n / SQ_CK) * n_samples + k]
+  unsigned long long* applied;  // map applications carried out
 };
+
+// An orbit that comes back to an iterate bit for bit repeats from there (the
+// map is a function of q's bits alone), and inside the set orbits do, after
+// 5-15 steps.  The forward pass compares each iterate with the one before
+// and with a marked one up to ORBIT_WINDOW steps back; on a match it leaves
+// out the whole periods that remain and adds their log|q'| increments, kept
+// since the mark, in the order the steps would have.  Every result keeps its
+// bits.  The kept orbit of the adjoint is filled in only for the few such
+// samples that have a gradient (the others saturate).  Energy + gradient
+// call of 200k samples, 64/16 roots, 30 iterations: 1380 -> 380 us (the
+// forward kernel 1290 -> 290).
+template <class T>
+struct OrbitWatch {
+  V4<T> mark;
+  int since;   // steps since the mark
+  int period;  // of the repeat found (0: none)
+  int at, skip;  // the steps [at, at + skip) left out
+};
+
+template <class T>
+__device__ __forceinline__ void watch_start(OrbitWatch<T>& w, const V4<T>& q) {
+  w.mark = q;
+  w.since = w.period = w.at = w.skip = 0;
+}
+
+__device__ __forceinline__ bool v4same(const V4<float>& a, const V4<float>& b) {
+  return __float_as_int(a.w) == __float_as_int(b.w) && __float_as_int(a.x) == __float_as_int(b.x) &&
+         __float_as_int(a.y) == __float_as_int(b.y) && __float_as_int(a.z) == __float_as_int(b.z);
+}
+__device__ __forceinline__ bool v4same(const V4<double>& a, const V4<double>& b) {
+  return same_bits(Q{a.w, a.x, a.y, a.z}, Q{b.w, b.x, b.y, b.z});
+}
+
+// After step n of an orbit that goes on (from `before` to q, log|q'| grown by
+// inc); incs is the thread's column of increments, `stride` apart.
+template <class T>
+__device__ __forceinline__ void watch_step(OrbitWatch<T>& w, const V4<T>& before, const V4<T>& q,
+                                           T inc, int max_it, T* incs, int stride, T& L, int& n) {
+  if (w.period) return;
+  incs[w.since * stride] = inc;
+  w.since++;
+  const int p = v4same(q, before) ? 1 : v4same(q, w.mark) ? w.since : 0;
+  if (p) {
+    w.period = p;
+    w.at = n;
+    w.skip = (max_it - n) / p * p;
+    const T* last = incs + (w.since - p) * stride;
+    for (int k = 0, j = 0; k < w.skip; k++, j = j + 1 < p ? j + 1 : 0) L += last[j * stride];
+    n += w.skip;
+  } else if (w.since >= mark_gap(n)) {
+    w.mark = q;
+    w.since = 0;
+  }
+}
 
 // Forward pass with lane refill: every lane iterates its own sample and takes
 // the next unclaimed one (a warp-aggregated atomic on *claim) as soon as its
@@ -1066,6 +1121,7 @@ __device__ __forceinline__ void sq_fwd_body(
     const double* __restrict__ target, long long n_samples, double slice, int max_it,
     double escape, double d_sat, unsigned long long* __restrict__ claim, const SqFwdOut<T>& o) {
   extern __shared__ unsigned char sh_raw[];
+  __shared__ T incs[ORBIT_WINDOW][SQF_T];
   const int nr = nt + nb;
   T* rp = reinterpret_cast<T*>(sh_raw);  // 4 nr
   T* ep = rp + 4 * nr;                   // nr
@@ -1076,6 +1132,8 @@ __device__ __forceinline__ void sq_fwd_body(
   const T esc = (T)escape, dsat = (T)d_sat;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
+  OrbitWatch<T> watch{};
+  unsigned applied = 0;
 
   // the sample's value, residual and (gradient pass) seed
   auto finish = [&](long long k, const V4<T>& q, T L, int n) {
@@ -1102,6 +1160,8 @@ __device__ __forceinline__ void sq_fwd_body(
         o.seed_q[k] = v4scale(q, kq / m);  // d/dq_N of d: (dd/dm) q_N / m
         o.seed_L[k] = -db * dval;
         key = n;
+        for (int j = watch.at; j < watch.at + watch.skip; j++)
+          o.ck[(long long)j * n_samples + k] = o.ck[(long long)(j - watch.period) * n_samples + k];
       }
     }
     o.keys[k] = key;
@@ -1128,6 +1188,7 @@ __device__ __forceinline__ void sq_fwd_body(
           q = V4<T>{(T)xyz[3 * k], (T)xyz[3 * k + 1], (T)xyz[3 * k + 2], (T)slice};
           L = T(0);
           n = 0;
+          watch_start(watch, q);
           if (sqrt(v4dot(q, q)) < esc && n < max_it)
             live = true;
           else
@@ -1140,17 +1201,24 @@ __device__ __forceinline__ void sq_fwd_body(
     if (live) {
       if (GRAD && n % SQ_CK == 0) o.ck[(long long)(n / SQ_CK) * n_samples + k] = q;
       T lg;
+      const V4<T> before = q;
       q = sq_apply<T, M>(rp, ep, nt, nb, s, q, &lg, nullptr, nullptr, nullptr, nullptr);
-      L += lg + T(0.5) * log(v4dot(q, q));
+      const T inc = lg + T(0.5) * log(v4dot(q, q));
+      L += inc;
       n++;
+      applied++;
       // 10 * FLT_MIN exit of the field loop
       const T m = sqrt(v4dot(q, q));
+      if (m < esc && n < max_it && !(m < T(1.1754943508e-37)))
+        watch_step(watch, before, q, inc, max_it, &incs[0][threadIdx.x], SQF_T, L, n);
       if (!(m < esc && n < max_it) || m < T(1.1754943508e-37)) {
         finish(k, q, L, n);
         live = false;
       }
     }
   }
+  applied = __reduce_add_sync(0xffffffffu, applied);
+  if (lane == 0 && applied) atomicAdd(o.applied, (unsigned long long)applied);
 }
 
 // The FP32 form is chosen once per launch, so that each form's root loop is
@@ -1264,6 +1332,7 @@ __device__ __forceinline__ void sq_fwd2_body(
   V4<T> q[2] = {{T(0), T(0), T(0), T(0)}, {T(0), T(0), T(0), T(0)}};
   T L[2] = {T(0), T(0)};
   int n[2] = {0, 0};
+  unsigned applied = 0;
   for (;;) {
 #pragma unroll
     for (int sl = 0; sl < 2; sl++) {
@@ -1306,6 +1375,7 @@ __device__ __forceinline__ void sq_fwd2_body(
       q[sl] = qn;
       L[sl] += (sl ? lgb : lga) + T(0.5) * log(v4dot(qn, qn));
       n[sl]++;
+      applied++;
       const T m = sqrt(v4dot(qn, qn));
       if (!(m < esc && n[sl] < max_it) || m < T(1.1754943508e-37)) {
         finish(k[sl], qn, L[sl], n[sl]);
@@ -1313,6 +1383,8 @@ __device__ __forceinline__ void sq_fwd2_body(
       }
     }
   }
+  applied = __reduce_add_sync(0xffffffffu, applied);
+  if (lane == 0 && applied) atomicAdd(o.applied, (unsigned long long)applied);
 }
 
 // The FP32 form is chosen once per launch (straight-line root loops).
@@ -1340,7 +1412,6 @@ __global__ void __launch_bounds__(SQF_T) sq_fwd2_kernel(
 // max_it - N so that long orbits come first: hist[bucket * nchunks + chunk].
 __global__ void __launch_bounds__(SQC_T) sq_chunk_kernel(const double* __restrict__ contrib,
                                                          const int* __restrict__ keys,
-                                                         const int* __restrict__ iters,
                                                          long long n, int max_it, int nchunks,
                                                          int* __restrict__ hist,
                                                          double* __restrict__ partials, int slots,
@@ -1352,12 +1423,11 @@ __global__ void __launch_bounds__(SQC_T) sq_chunk_kernel(const double* __restric
   for (int b = t; b <= max_it; b += SQC_T) h[b] = 0;
   __syncthreads();
   double e = 0.0, bad = 0.0;
-  unsigned long long apps = 0, steps = 0;  // map applications (forward), orbit steps (adjoint)
+  unsigned long long steps = 0;  // orbit steps of the adjoint
   for (int i = t; i < SQ_CH; i += SQC_T) {
     const long long k = (long long)c * SQ_CH + i;
     if (k >= n) break;
     e += contrib[k];
-    apps += (unsigned long long)iters[k];
     if (keys) {
       const int key = keys[k];
       if (key == -2) bad += 1.0;
@@ -1367,12 +1437,8 @@ __global__ void __launch_bounds__(SQC_T) sq_chunk_kernel(const double* __restric
       }
     }
   }
-  apps = __reduce_add_sync(0xffffffffu, (unsigned)apps);
   steps = __reduce_add_sync(0xffffffffu, (unsigned)steps);
-  if ((t & 31) == 0 && (apps | steps)) {
-    atomicAdd(&work[0], apps);
-    atomicAdd(&work[1], steps);
-  }
+  if ((t & 31) == 0 && steps) atomicAdd(&work[1], steps);
   red_e[t] = e;
   red_b[t] = bad;
   __syncthreads();
@@ -1994,6 +2060,10 @@ __device__ __forceinline__ void sq_fwd_batch_body(
     const SqItem* __restrict__ items, const int* __restrict__ chunk_item, long long n_flat,
     unsigned long long* __restrict__ claim, SqFwdOut<float> o) {
   using T = float;
+  __shared__ T incs[ORBIT_WINDOW][SQF_T];
+  OrbitWatch<T> watch{};
+  unsigned applied = 0;
+  T s = T(0);
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   long long k = 0;       // flat sample
@@ -2023,6 +2093,8 @@ __device__ __forceinline__ void sq_fwd_batch_body(
         o.seed_q[kf] = v4scale(qf, kq / m);
         o.seed_L[kf] = -db * dval;
         key = nf;
+        for (int j = watch.at; j < watch.at + watch.skip; j++)
+          o.ck[(long long)j * n_flat + kf] = o.ck[(long long)(j - watch.period) * n_flat + kf];
       }
     }
     o.keys[kf] = key;
@@ -2046,6 +2118,8 @@ __device__ __forceinline__ void sq_fwd_batch_body(
                       (T)it->slice};
             L = T(0);
             n = 0;
+            s = (T)exp(it->params[5 * (it->nt + it->nb)]);
+            watch_start(watch, q);
             if (sqrt(v4dot(q, q)) < (T)it->escape && n < it->max_it)
               live = true;
             else
@@ -2059,19 +2133,25 @@ __device__ __forceinline__ void sq_fwd_batch_body(
     if (live) {
       if (n % SQ_CK == 0) o.ck[(long long)(n / SQ_CK) * n_flat + k] = q;
       const int nr = it->nt + it->nb;
-      const T s = (T)exp(it->params[5 * nr]);
       T lg;
+      const V4<T> before = q;
       q = sq_apply<T, M>(it->rp, it->rp + 4 * nr, it->nt, it->nb, s, q, &lg, nullptr, nullptr,
                       nullptr, nullptr);
-      L += lg + T(0.5) * log(v4dot(q, q));
+      const T inc = lg + T(0.5) * log(v4dot(q, q));
+      L += inc;
       n++;
+      applied++;
       const T m = sqrt(v4dot(q, q));
+      if (m < (T)it->escape && n < it->max_it && !(m < T(1.1754943508e-37)))
+        watch_step(watch, before, q, inc, it->max_it, &incs[0][threadIdx.x], SQF_T, L, n);
       if (!(m < (T)it->escape && n < it->max_it) || m < T(1.1754943508e-37)) {
         finish(k, q, L, n);
         live = false;
       }
     }
   }
+  applied = __reduce_add_sync(0xffffffffu, applied);
+  if (lane == 0 && applied) atomicAdd(o.applied, (unsigned long long)applied);
 }
 
 // The FP32 form is chosen once per launch (straight-line root loops).
@@ -2422,7 +2502,7 @@ template <class T>
 cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const double* xyz,
                       const double* target, long long n, double slice, int max_it, double escape,
                       double d_sat, unsigned char* scr, const SqLayout& L, int* iters, int sms,
-                      cudaStream_t s, int* launches, long long steps_hint) {
+                      cudaStream_t s, int* launches) {
   const int nr = nt + nb;
   unsigned long long* claim = reinterpret_cast<unsigned long long*>(scr + L.claim);
   int* total = reinterpret_cast<int*>(scr + L.total);
@@ -2432,6 +2512,7 @@ cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const dou
   o.keys = reinterpret_cast<int*>(scr + L.keys);
   o.iters = iters ? iters : reinterpret_cast<int*>(scr + L.iters);
   unsigned long long* work = reinterpret_cast<unsigned long long*>(scr + L.work);
+  o.applied = work;
   if (grad) {
     o.seed_q = reinterpret_cast<V4<T>*>(scr + L.seed_q);
     o.seed_L = reinterpret_cast<T*>(scr + L.seed_L);
@@ -2448,29 +2529,18 @@ cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const dou
   else
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sq_fwd_kernel<T, false>, SQF_T, sh_roots);
   if (e != cudaSuccess) return e;
-  // Blocks per SM.  The kernel ends when the lane with the most orbit steps
-  // ends, so the grid is sized from the orbit steps of the call: with as
-  // many lanes as total steps / max_it, a lane runs about one full-length
-  // orbit (or its equivalent in short ones) and no lane is left with two
-  // full-length orbits, while each extra warp costs issue slots.  On the
-  // differentiation workload (200k samples, 30 iterations, 3.06 M steps,
-  // 49% of the orbits at the cap; forward kernel, ms) 2 blocks per SM 1.22,
-  // 3 0.96, 4 1.01, 5 0.96, 6 0.83, 8 1.03: 6 is the first count with a lane
-  // per full-length orbit.  The steps are those of an earlier call on the
-  // same samples (steps_hint), else half the iteration cap per sample (a
-  // lane per two samples); at least 3 blocks per SM.  FP64 (bound by the
-  // FP64 pipe rather than by the longest lane) keeps about four samples per
-  // lane.
+  // Blocks per SM: in FP32 as many as stay resident.  With the settled
+  // orbits cut short a sample takes about 4 map applications and the longest
+  // lanes are those few samples that do not settle, so more lanes only fill
+  // issue slots (energy + gradient call, us, at 3 / 4 / 5 / all blocks per
+  // SM: 200k samples, 64/16 roots 421 / 383 / 381 / 380; 100k, 32/16 roots
+  // 256 / 266 / 230 / 248; 50k and fewer samples within 1%).  FP64 (bound by
+  // the FP64 pipe) keeps about four samples per lane.
   const long long lanes_per_sm = (long long)sms * SQF_T;
   const int fixed = g_sq_fwd_blocks.load(std::memory_order_relaxed);
   long long want = std::max<long long>(3, ((n + 3) / 4 + lanes_per_sm - 1) / lanes_per_sm);
-  if (fixed > 0) {
-    want = fixed;
-  } else if (std::is_same<T, float>::value && max_it > 0) {
-    const long long steps = steps_hint > 0 ? steps_hint : (n * max_it + 1) / 2;
-    const long long lanes = (steps + max_it - 1) / max_it;
-    want = std::max<long long>(3, (lanes + lanes_per_sm - 1) / lanes_per_sm);
-  }
+  if (fixed > 0) want = fixed;
+  else if (std::is_same<T, float>::value) want = per_sm;
   const long long need = (n + SQF_T - 1) / SQF_T;
   const int fblocks = (int)std::max<long long>(
       1, std::min<long long>((long long)sms * std::min<long long>(std::max(per_sm, 1), want), need));
@@ -2489,7 +2559,7 @@ cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const dou
                                                              max_it, escape, d_sat, claim, o);
   }
   int* hist = grad ? reinterpret_cast<int*>(scr + L.hist) : nullptr;
-  sq_chunk_kernel<<<L.nchunks, SQC_T, 0, s>>>(o.contrib, grad ? o.keys : nullptr, o.iters, n,
+  sq_chunk_kernel<<<L.nchunks, SQC_T, 0, s>>>(o.contrib, grad ? o.keys : nullptr, n,
                                               max_it, L.nchunks, hist, partials, L.slots, 0, work);
   *launches = 3;
   int bwd_blocks = L.nbwd;  // rows of backward partials written
@@ -2645,20 +2715,14 @@ cudaError_t launch_sq_energy_batch(const SqBatchReq* r, int K, void* scratch, do
   o.seed_q = reinterpret_cast<V4<float>*>(scr + L.seed_q);
   o.seed_L = reinterpret_cast<float*>(scr + L.seed_L);
   o.ck = reinterpret_cast<V4<float>*>(scr + L.ck);
-  // persistent forward grid: as the single request's first call, a lane per
-  // two samples of the batch (at least 3 blocks per SM, at most the resident
-  // count), fewer when the batch is small
+  o.applied = work;
+  // persistent forward grid: the resident blocks, as the single call
   int per_sm = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sq_fwd_batch_kernel, SQF_T, 0)))
     return e;
   const long long need = (L.n_flat + SQF_T - 1) / SQF_T;
-  long long total_n = 0;
-  for (int i = 0; i < K; i++) total_n += r[i].n;
-  const long long lanes_per_sm = (long long)sms * SQF_T;
-  const long long want = std::min<long long>(
-      std::max(per_sm, 1),
-      std::max<long long>(3, ((total_n + 1) / 2 + lanes_per_sm - 1) / lanes_per_sm));
-  const int fblocks = (int)std::max<long long>(1, std::min<long long>((long long)sms * want, need));
+  const int fblocks = (int)std::max<long long>(
+      1, std::min<long long>((long long)sms * std::max(per_sm, 1), need));
   sq_fwd_batch_kernel<<<fblocks, SQF_T, 0, s>>>(d_items, d_chunk_item, L.n_flat, claim, o);
   n_launch++;
   // per item: chunk sums and histogram, the sort's scan and scatter
@@ -2666,7 +2730,7 @@ cudaError_t launch_sq_energy_batch(const SqBatchReq* r, int K, void* scratch, do
     const long long s0 = L.s0[(size_t)i];
     int* hist = reinterpret_cast<int*>(scr + L.hist[(size_t)i]);
     sq_chunk_kernel<<<(unsigned)L.nchunks[(size_t)i], SQC_T, 0, s>>>(
-        o.contrib + s0, o.keys + s0, o.iters + s0, r[i].n, r[i].max_it, (int)L.nchunks[(size_t)i],
+        o.contrib + s0, o.keys + s0, r[i].n, r[i].max_it, (int)L.nchunks[(size_t)i],
         hist, items[(size_t)i].partials, L.slots[(size_t)i], 0, work);
     sq_scan_kernel<<<1, 1024, 0, s>>>(hist, (long long)(r[i].max_it + 1) * L.nchunks[(size_t)i],
                                       items[(size_t)i].total);
@@ -2741,7 +2805,7 @@ cudaError_t launch_sq_energy(bool fp64, bool grad, const double* params, int nt,
                              const double* xyz, const double* target, long long n, double slice,
                              int max_it, double escape, double d_sat, void* scratch,
                              double** out, int* iters, cudaStream_t s, int* launches,
-                             unsigned long long** work, long long steps_hint) {
+                             unsigned long long** work) {
   const int sms = sm_count();
   const SqLayout L = sq_layout(fp64, grad, n, max_it, nt, nb, sms);
   unsigned char* scr = static_cast<unsigned char*>(scratch);
@@ -2749,9 +2813,9 @@ cudaError_t launch_sq_energy(bool fp64, bool grad, const double* params, int nt,
   *work = reinterpret_cast<unsigned long long*>(scr + L.work);
   if (fp64)
     return sq_launch<double>(grad, params, nt, nb, xyz, target, n, slice, max_it, escape, d_sat,
-                             scr, L, iters, sms, s, launches, steps_hint);
+                             scr, L, iters, sms, s, launches);
   return sq_launch<float>(grad, params, nt, nb, xyz, target, n, slice, max_it, escape, d_sat, scr,
-                          L, iters, sms, s, launches, steps_hint);
+                          L, iters, sms, s, launches);
 }
 
 }  // namespace qj
