@@ -86,6 +86,16 @@ int qjg_energy_last_work(qjg_ctx* ctx, int64_t* applications, int64_t* steps);
 #define QJG_CRM_SIN 2
 #define QJG_CRM_COS 3
 #define QJG_CRM_ACOS 4
+/* ... and the integer-pipe functions of the plain form's polar power
+ * (arguments within their ranges: positive normal numbers; |log x| < 100,
+ * 2^-60 < |exp's x| < 700, 2^-20 < sin/cos's x < 2^11, |acos's x| < 1 - 2^-17). */
+#define QJG_FX_EXP 5
+#define QJG_FX_LOG 6
+#define QJG_FX_SIN 7
+#define QJG_FX_COS 8
+#define QJG_FX_ACOS 9
+#define QJG_FX_SQRT 10
+#define QJG_FX_RCP 11
 int qjg_crmath_eval(int fn, const double* d_x, double* d_y, int64_t n, void* stream);
 
 /* FP32 FMA-pipe probe: runs a kernel of independent FMA chains on every SM

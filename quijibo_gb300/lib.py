@@ -17,7 +17,10 @@ QJG_OK, QJG_ERR_ARG, QJG_ERR_CUDA, QJG_ERR_NOMEM, QJG_ERR_HANDLE, QJG_ERR_CAPACI
 QJG_FP64, QJG_FP32, QJG_FP32_REFINE = 0, 1, 2
 QJG_REFINE_POW, QJG_REFINE_INT = 0, 1
 QJG_LIBM_DEVICE, QJG_LIBM_CR = 0, 1
-CRM_FUNCTIONS = ("exp", "log", "sin", "cos", "acos")  # qjg_crmath_eval's fn order
+# qjg_crmath_eval's fn order: the correctly rounded functions, then the
+# integer-pipe ones of the polar power
+CRM_FUNCTIONS = ("exp", "log", "sin", "cos", "acos")
+FX_FUNCTIONS = ("fx_exp", "fx_log", "fx_sin", "fx_cos", "fx_acos", "fx_sqrt", "fx_rcp")
 
 _dp = C.POINTER(C.c_double)
 _fp = C.POINTER(C.c_float)
@@ -487,8 +490,9 @@ def set_field32_pairs(on):
 
 def crmath_eval(name, d_x, d_y, n, stream=None):
     """y[i] = f(x[i]) on the device with the correctly rounded FP64 function
-    `name` (one of CRM_FUNCTIONS) of the QJG_LIBM_CR form; device pointers."""
-    rc = load().qjg_crmath_eval(CRM_FUNCTIONS.index(name), C.c_void_p(d_x), C.c_void_p(d_y),
+    `name` (one of CRM_FUNCTIONS) of the QJG_LIBM_CR form, or an integer-pipe
+    one (FX_FUNCTIONS); device pointers."""
+    rc = load().qjg_crmath_eval((CRM_FUNCTIONS + FX_FUNCTIONS).index(name), C.c_void_p(d_x), C.c_void_p(d_y),
                                 int(n), C.c_void_p(stream or 0))
     if rc != 0:
         raise QjgError("qjg_crmath_eval failed (%d)" % rc)
