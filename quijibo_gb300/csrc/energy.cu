@@ -34,8 +34,6 @@ namespace {
 
 using namespace q64;
 
-constexpr int EN_T = 128;  // threads per block
-
 // QUATERNION::log, QUATERNION.cpp:352-365.
 __device__ __forceinline__ Q qlog(const Q& q) {
   const double qm = mag(q);
@@ -457,33 +455,180 @@ __device__ __noinline__ void grad_terms_ext(const MapParams& m, const Q q0, bool
   warp_accum(acc, s_bulkb_x, c_bulk_bx);
 }
 
-// Block b takes a contiguous range of voxels, EN_T at a time.  Every voxel's
-// map, field, score and d/d log s term are computed in the first step.  The
-// per-parameter terms are skipped where they are exact zeros (saturated tanh
-// or zero weight, with every intermediate provably in range); a warp with at
-// least 24 voxels needing them computes them at once from the factors it
-// holds (16.2 / 15.0 / 14.5 ms per pass at 8 / 16 / 24 on the 97^3
-// objective benchmark), sparser ones queue their voxels in shared memory, in
-// voxel order, to be re-evaluated and computed EN_T at a time in full warps.
-template <bool POW_REF>
-__global__ void __launch_bounds__(EN_T, 4) tanh_grad_kernel(const __grid_constant__ MapParams m,
-                                                         const GridParams g, const WeightGrid wg,
-                                                         const double* __restrict__ weights,
-                                                         int max_it, double alpha, double thr,
-                                                         double* __restrict__ field,
-                                                         double* __restrict__ partials, int slots) {
-  extern __shared__ double acc_sh[];  // [EN_T / 32][slots]
-  __shared__ long long queue[2 * EN_T];
-  __shared__ int queued, wcount[EN_T / 32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* acc = acc_sh + warp * slots;
-  for (int k = threadIdx.x; k < (EN_T / 32) * slots; k += EN_T) acc_sh[k] = 0.0;
-  if (threadIdx.x == 0) queued = 0;
-  __syncthreads();
+// One application of the map from q0 (max_it = 1, the optimizer's form): T, B
+// and the overflow test as eval_voxel, with what the gradient needs of each
+// root in Pf and Lg and without the suffix products: an overflow there needs
+// factors whose magnitudes spread over more than 2^600, and only such voxels
+// evaluate them (into Sf).
+__device__ __forceinline__ void eval_one(const MapParams& m, const Q& q0, Q* Pf, double2* Lg,
+                                         Q* Sf, Voxel& v) {
+  const int nt = m.nt, nb = m.nb;
+  v.q0 = q0;
+  v.T = Q{1, 0, 0, 0};
+  v.B = Q{1, 0, 0, 0};
+  v.its = 0;
+  v.over = false;
+  v.iterated = false;
+  v.spread = 0;
+  v.bases_ok = true;
+  v.mg = mag(q0);
+  if (v.mg < 1e-8 || !(v.mg < 20.0)) return;  // "if we hit the origin, move on"; escaped
+  v.iterated = true;
+  v.its = 1;
+#pragma unroll 1
+  for (int side = 0; side < 2; side++) {
+    const int lo = side ? nt : 0, hi = side ? nt + nb : nt;
+    Q acc_q = {1, 0, 0, 0};
+#pragma unroll 1
+    for (int i = lo; i < hi; i++) {
+      const Q d{sub(q0.w, m.r64[i][0]), sub(q0.x, m.r64[i][1]), sub(q0.y, m.r64[i][2]),
+                sub(q0.z, m.r64[i][3])};
+      PowLog pl;
+      const Q P = qpow<true>(d, m.e64[i], &pl);
+      Pf[i] = P;
+      Lg[i] = make_double2(pl.l, pl.a);
+      acc_q = (i == lo) ? P : qmul(acc_q, P);
+      // |log2 |P|^2|, and d of moderate size and away from 1, from exponents
+      v.spread += abs(2 * ilog2_bits(pl.amp));
+      const unsigned big = max(max(exp_field(d.x), exp_field(d.y)) & 0x7ffu,
+                               max(exp_field(d.z) & 0x7ffu, exp_field(sub(d.w, 1.0)) & 0x7ffu));
+      v.bases_ok = v.bases_ok && fabs(pl.l) < 46.0 && big > 1023u - 33u;
+    }
+    if (side == 0)
+      v.T = acc_q;
+    else if (nb > 0)
+      v.B = acc_q;
+  }
+  bool suffix_ok = true;
+  if (!(v.spread <= 600)) {
+#pragma unroll 1
+    for (int side = 0; side < 2; side++) {
+      const int lo = side ? nt : 0, hi = side ? nt + nb : nt;
+      if (hi == lo) continue;
+      Sf[hi - 1] = Pf[hi - 1];
+#pragma unroll 1
+      for (int i = hi - 2; i >= lo; i--) Sf[i] = qmul(Pf[i], Sf[i + 1]);
+      suffix_ok = suffix_ok && isfinite(Sf[lo].w) && isfinite(Sf[lo].x) && isfinite(Sf[lo].y) &&
+                  isfinite(Sf[lo].z);
+    }
+  }
+  const Q& T = v.T;
+  const Q& B = v.B;
+  Q q = nb > 0 ? qdiv(T, B) : T;
+  v.over = !suffix_ok || !isfinite(T.w) || !isfinite(T.x) || !isfinite(T.y) || !isfinite(T.z) ||
+           (nb > 0 && (!isfinite(B.w) || !isfinite(B.x) || !isfinite(B.y) || !isfinite(B.z) ||
+                       isinf(norm2(B)))) ||
+           !isfinite(q.w) || !isfinite(q.x) || !isfinite(q.y) || !isfinite(q.z);
+  q = qscale(q, m.scale);
+  v.mg = mag(q);
+  if (isinf(v.mg) || isnan(v.mg)) v.over = true;
+}
+
+__device__ __forceinline__ Q fconj(const Q& a) { return Q{a.w, -a.x, -a.y, -a.z}; }
+__device__ __forceinline__ double fdot(const Q& a, const Q& b) {
+  return fma(a.z, b.z, fma(a.y, b.y, fma(a.x, b.x, mul(a.w, b.w))));
+}
+
+// The per-parameter terms of one voxel of eval_one, added to the lane's own
+// sums (sums[i]: root i's exponent; *bulk_t, *bulk_b: the power scalars).
+// The same gradient as grad_terms, with each root's inner product turned
+// around: <R, L (P log d) S / B> = <conj(L) R conj(S / B), P log d>, where
+// conj(L) R B / |B|^2 is a running product; and the bottom roots' formula
+// T / (-L Y S) with Y = P / log d, |L P S| = |B|:
+//   -<S conj(T) R L, log d conj(P)> / |B|^2.
+// A root's exponent and its power scalar differ by a factor only, so one
+// inner product serves both: 52 FP64 instructions a root where grad_terms
+// issues about 400 (two passes of five products, its own logarithm).  Sums
+// stay in the lane until its voxels are done (a warp sum per root and voxel
+// was 5 more).  For voxels whose intermediates are moderate (the caller's
+// test); the others take grad_terms.
+__device__ __forceinline__ void terms_one(const MapParams& m, const Voxel& v, const Q& R,
+                                          double dSdF, double RR, const Q* Pf, const double2* Lg,
+                                          Q* Sf, double* sums, double& bulk_t, double& bulk_b,
+                                          double& bad) {
+  const int nt = m.nt, nb = m.nb;
+  const double c0 = mul(dSdF, RR);
+  const double ib = nb > 0 ? __ddiv_rn(1.0, fnorm2(v.B)) : 1.0;
+#pragma unroll 1
+  for (int side = 0; side < 2; side++) {
+    const int lo = side ? nt : 0, hi = side ? nt + nb : nt;
+    if (hi == lo) continue;
+    Q S = Pf[hi - 1];
+#pragma unroll 1
+    for (int i = hi - 2; i >= lo; i--) {  // Sf[i]: the product after root i
+      Sf[i] = S;
+      if (i > lo) S = fmul(Pf[i], S);
+    }
+    // top: conj(L) R B / |B|^2; bottom: conj(T) R L
+    Q H = side ? fmul(fconj(v.T), R) : nb > 0 ? fmul(R, v.B) : R;
+    H = qscale(H, mul(c0, ib));
+#pragma unroll 1
+    for (int i = lo; i < hi; i++) {
+      const Q P = Pf[i];
+      const double2 pl = Lg[i];  // log|d|, angle / |v|
+      const Q d{sub(v.q0.w, m.r64[i][0]), sub(v.q0.x, m.r64[i][1]), sub(v.q0.y, m.r64[i][2]),
+                sub(v.q0.z, m.r64[i][3])};
+      const Q lg{pl.x, mul(pl.y, d.x), mul(pl.y, d.y), mul(pl.y, d.z)};
+      double t;
+      if (side == 0) {
+        const Q V = i < hi - 1 ? fmul(H, fconj(Sf[i])) : H;
+        t = fdot(V, fmul(P, lg));
+        if (i < hi - 1) H = fmul(fconj(P), H);
+      } else {
+        const Q W = i < hi - 1 ? fmul(Sf[i], H) : H;
+        t = -fdot(W, fmul(lg, fconj(P)));
+        if (i < hi - 1) H = fmul(H, P);
+      }
+      if (isnan(t) || isinf(t)) {
+        bad += side == 0 ? 2.0 : (m.sigma[1] > 0.0 ? 1.0 : 0.0) + (m.ep[i] < 1e-8 ? 0.0 : 1.0);
+      } else if (side == 0) {
+        sums[i] += t;  // times sigma_t at the end
+        bulk_t = fma(m.ep[i], t, bulk_t);
+      } else {
+        sums[i] += t;
+        if (!(m.ep[i] < 1e-8)) bulk_b = fma(m.ep[i], t, bulk_b);
+      }
+    }
+  }
+}
+
+// A block is one warp with a contiguous range of `per` voxels, 32 at a time
+// (the hardware hands the ranges out, so SMs whose voxels saturate take more
+// of them: with one range per resident block the SMs were active for 77% of
+// the launch).  Every voxel's map, field, score and d/d log s term are
+// computed in the first step.  The per-parameter terms are skipped where they
+// are exact zeros (saturated tanh or zero weight, with every intermediate
+// provably in range); a step with at least 24 voxels needing them computes
+// them at once from the factors it holds, sparser ones queue their voxels, in
+// voxel order, to be re-evaluated and computed 32 at a time.
+// ONE: max_it = 1, eval_one and terms_one; else eval_voxel and grad_terms.
+// FP64-pipe bound; objective pass of a 97^3 grid, 12 / 6 roots: 17.7 ms
+// before the integer-pipe power, 13.2 with it, 4.9 in this form (25^3: 0.92,
+// 0.77, 0.29 ms).
+template <bool ONE>
+__global__ void __launch_bounds__(32, 16) tanh_grad_kernel(const __grid_constant__ MapParams m,
+                                                        const GridParams g, const WeightGrid wg,
+                                                        const double* __restrict__ weights,
+                                                        int max_it, double alpha, double thr,
+                                                        double* __restrict__ field,
+                                                        double* __restrict__ partials, int slots,
+                                                        long long per) {
+  extern __shared__ double acc[];  // [slots]
+  __shared__ long long queue[64];
+  const int lane = threadIdx.x;
+  for (int k = lane; k < slots; k += 32) acc[k] = 0.0;
+  __syncwarp();
+  int queued = 0;
   Q Pf[QJ_MAX_ROOTS];  // last application's factors (local memory)
   Q Sf[QJ_MAX_ROOTS];  // their suffix products
   int Pe[QJ_MAX_ROOTS], Se[QJ_MAX_ROOTS];  // their exponents on the extended path
+  double2 Lg[ONE ? QJ_MAX_ROOTS : 1];      // the factors' logarithms
+  double sums[ONE ? QJ_MAX_ROOTS : 1];     // the lane's exponent terms
   const int nt = m.nt, nb = m.nb;
+  if (ONE)
+    for (int i = 0; i < nt + nb; i++) sums[i] = 0.0;
+  double bulk_t = 0, bulk_b = 0, bad = 0;
+  double s_exp = 0, s_sco = 0, s_ov = 0, s_ba = 0;
   const long long N = (long long)g.X * g.Y * g.Z;
   const double logs = log(m.scale);
   const int s_score = 3 + nt + nb, s_over = s_score + 1, s_bad = s_score + 2;
@@ -496,7 +641,6 @@ __global__ void __launch_bounds__(EN_T, 4) tanh_grad_kernel(const __grid_constan
     const double e = fabs(m.ep[i]);
     k_ok = k_ok && (e == 0.0 || (e >= 1e-10 && e <= 1e10));
   }
-  const long long per = (N + gridDim.x - 1) / gridDim.x;
   const long long lo_b = (long long)blockIdx.x * per;
   const long long hi_b = lo_b + per < N ? lo_b + per : N;
   auto cell = [&](long long idx, double* p) {
@@ -504,27 +648,56 @@ __global__ void __launch_bounds__(EN_T, 4) tanh_grad_kernel(const __grid_constan
     const int z = (int)(idx / ((long long)g.X * g.Y));
     cell_center(g, x, y, z, p);
   };
-  // the queued voxels' terms: each thread re-evaluates one voxel's map
+  // whether every intermediate of a voxel's terms stays in range: the
+  // factors' magnitudes spread over at most 2^300, every q0 - root moderate
+  // and away from 1, every k moderate
+  auto moderate = [&](const Voxel& v, const Q& R) {
+    const double r2 = qdot(R, R), b2 = norm2(v.B);
+    return k_ok && v.bases_ok && v.spread <= 300 && r2 > 1e-260 && r2 < 1e260 && b2 > 1e-130 &&
+           b2 < 1e130;
+  };
+  // the terms of this step's voxels (ok), one per lane
+  auto terms = [&](const Voxel& v, bool ok, const Q& R, double dSdF, double RR) {
+    bool general = ok;
+    if (ONE) {
+      const bool easy = ok && moderate(v, R);
+      if (easy) terms_one(m, v, R, dSdF, RR, Pf, Lg, Sf, sums, bulk_t, bulk_b, bad);
+      general = ok && !easy;
+      if (!__any_sync(0xffffffffu, general)) return;
+      if (general) {  // the suffix products that grad_terms reads
+        for (int side = 0; side < 2; side++) {
+          const int lo = side ? nt : 0, hi = side ? nt + nb : nt;
+          if (hi == lo) continue;
+          Sf[hi - 1] = Pf[hi - 1];
+#pragma unroll 1
+          for (int i = hi - 2; i >= lo; i--) Sf[i] = qmul(Pf[i], Sf[i + 1]);
+        }
+      }
+    }
+    grad_terms<true>(m, v, general, R, dSdF, RR, Pf, Sf, acc, s_bad);
+  };
+  // the queued voxels' terms: each lane re-evaluates one voxel's map
   auto drain = [&](int count) {
-    const bool ok = threadIdx.x < count;
+    const bool ok = lane < count;
     Voxel v;
     Q R = {0, 0, 0, 0};
     double dSdF = 0, RR = 0;
     bool good = false;
     if (ok) {
       double p[3];
-      cell(queue[threadIdx.x], p);
-      eval_voxel<POW_REF, false>(m, Q{p[0], p[1], p[2], g.slice}, max_it, Pf, Sf, v);
+      cell(queue[lane], p);
+      const Q q0{p[0], p[1], p[2], g.slice};
+      if (ONE) eval_one(m, q0, Pf, Lg, Sf, v);
+      else eval_voxel<true, false>(m, q0, max_it, Pf, Sf, v);
       good = grad_setup(v, logs, alpha, thr, trilinear(wg, weights, p), R, dSdF, RR);
     } else {
       v.its = 0;
     }
-    grad_terms<POW_REF>(m, v, good, R, dSdF, RR, Pf, Sf, acc, s_bad);
+    terms(v, good, R, dSdF, RR);
   };
-  for (long long base = lo_b; base < hi_b; base += EN_T) {
-    const long long idx = base + threadIdx.x;
+  for (long long base = lo_b; base < hi_b; base += 32) {
+    const long long idx = base + lane;
     const bool live = idx < hi_b;
-    double c_exp = 0, c_score = 0, c_over = 0, c_band = 0;
     bool want = false, ext = false;
     Voxel v;
     v.over = false;
@@ -539,31 +712,24 @@ __global__ void __launch_bounds__(EN_T, 4) tanh_grad_kernel(const __grid_constan
       double p[3];
       cell(idx, p);
       q0 = Q{p[0], p[1], p[2], g.slice};
-      eval_voxel<POW_REF, true>(m, q0, max_it, Pf, Sf, v);
+      if (ONE) eval_one(m, q0, Pf, Lg, Sf, v);
+      else eval_voxel<true, true>(m, q0, max_it, Pf, Sf, v);
       double fval = 0.0;
       if (v.iterated || v.mg >= 1e-8) fval = log(v.mg);
-      if (!(mag(q0) < 1e-8) && v.over)
-        fval = ext_map<POW_REF>(m, q0, max_it, Pf, Pe, &Tx, &Bx);
+      if (!(mag(q0) < 1e-8) && v.over) fval = ext_map<true>(m, q0, max_it, Pf, Pe, &Tx, &Bx);
       if (field) field[idx] = fval;
       const double w = trilinear(wg, weights, p);
-      c_score = mul(-tanh(mul(alpha, fval)), w);
+      const double S0 = tanh(mul(alpha, fval));
+      s_sco += mul(-S0, w);
       {
-        const double S = tanh(mul(alpha, sub(fval, thr)));
-        c_exp = mul(mul(-alpha, w), sub(1.0, mul(S, S)));
+        const double S = thr == 0.0 ? S0 : tanh(mul(alpha, sub(fval, thr)));
+        s_exp += mul(mul(-alpha, w), sub(1.0, mul(S, S)));
       }
-      c_over = v.over ? 1.0 : 0.0;
+      s_ov += v.over ? 1.0 : 0.0;
       if (v.iterated && !v.over) {
-        Q& R = Rg;
-        double& RR = RRg;
-        if (grad_setup(v, logs, alpha, thr, w, R, dSdF, RR)) {
-          // dSdF = 0 makes every term dSdF * y an exact zero; y stays finite
-          // when the factors' magnitudes spread over at most 2^300, every
-          // q0 - root is moderate and away from 1 and every k is moderate
-          const double r2 = qdot(R, R), b2 = norm2(v.B);
-          const bool zero_terms = dSdF == 0.0 && k_ok && v.bases_ok && v.spread <= 300 &&
-                                  r2 > 1e-260 && r2 < 1e260 && b2 > 1e-130 && b2 < 1e130;
-          want = !zero_terms;
-        }
+        // dSdF = 0 makes every term dSdF * y an exact zero where y is finite
+        if (grad_setup(v, logs, alpha, thr, w, Rg, dSdF, RRg))
+          want = !(dSdF == 0.0 && moderate(v, Rg));
       } else if (v.iterated) {
         // the gradients' overflow pass, on the extended factors
         Rx = xdiv(Tx, Bx);
@@ -587,77 +753,75 @@ __global__ void __launch_bounds__(EN_T, 4) tanh_grad_kernel(const __grid_constan
           }
         }
       }
-      c_band = want ? 1.0 : 0.0;
+      s_ba += want ? 1.0 : 0.0;
     }
-    warp_accum(acc, 0, c_exp);
-    warp_accum(acc, s_score, c_score);
-    warp_accum(acc, s_over, c_over);
-    warp_accum(acc, s_band, c_band);
     if (__any_sync(0xffffffffu, ext))
       grad_terms_ext(m, q0, ext, Rx, Tx, Bx, dSdF, Pf, Pe, Sf, Se, acc, s_bulkb_x);
-    // a warp with many voxels needing their terms computes them now, from
-    // the factors it holds; the others append theirs to the queue, in voxel
-    // order, to be computed in full warps
-    unsigned bal = __ballot_sync(0xffffffffu, want);
+    const unsigned bal = __ballot_sync(0xffffffffu, want);
     if (__popc(bal) >= 24) {
-      grad_terms<POW_REF>(m, v, want, Rg, dSdF, RRg, Pf, Sf, acc, s_bad);
-      bal = 0;
-      want = false;
+      terms(v, want, Rg, dSdF, RRg);
+      continue;
     }
-    if (lane == 0) wcount[warp] = __popc(bal);
-    __syncthreads();
-    int off = queued;
-    for (int k = 0; k < warp; k++) off += wcount[k];
-    if (want) queue[off + __popc(bal & ((1u << lane) - 1u))] = idx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int tot = 0;
-      for (int k = 0; k < EN_T / 32; k++) tot += wcount[k];
-      queued += tot;
-    }
-    __syncthreads();
-    if (queued >= EN_T) {
-      drain(EN_T);
-      __syncthreads();
-      const int rest = queued - EN_T;
-      if (threadIdx.x < rest) queue[threadIdx.x] = queue[EN_T + threadIdx.x];
-      __syncthreads();
-      if (threadIdx.x == 0) queued = rest;
-      __syncthreads();
+    if (want) queue[queued + __popc(bal & ((1u << lane) - 1u))] = idx;
+    queued += __popc(bal);
+    __syncwarp();
+    if (queued >= 32) {
+      drain(32);
+      __syncwarp();
+      queued -= 32;
+      const long long moved = queue[32 + lane];
+      __syncwarp();
+      if (lane < queued) queue[lane] = moved;
+      __syncwarp();
     }
   }
   if (queued > 0) drain(queued);
-  __syncthreads();
-  for (int k = threadIdx.x; k < slots; k += EN_T) {
-    double s = 0;
-    for (int wv = 0; wv < EN_T / 32; wv++) s += acc_sh[wv * slots + k];
-    partials[(long long)blockIdx.x * slots + k] = s;
+  warp_accum(acc, 0, s_exp);
+  warp_accum(acc, s_score, s_sco);
+  warp_accum(acc, s_over, s_ov);
+  warp_accum(acc, s_band, s_ba);
+  if (ONE) {
+    warp_accum(acc, 1 + nb + nt, bulk_t);
+    warp_accum(acc, 2 + nb + nt, bulk_b);
+    warp_accum(acc, s_bad, bad);
+    for (int i = 0; i < nt; i++) warp_accum(acc, 1 + nb + i, mul(m.sigma[0], sums[i]));
+    if (m.sigma[1] > 0.0)
+      for (int j = 0; j < nb; j++) warp_accum(acc, 1 + j, mul(m.sigma[1], sums[nt + j]));
   }
+  __syncwarp();
+  for (int k = lane; k < slots; k += 32) partials[(long long)blockIdx.x * slots + k] = acc[k];
 }
 
-// Neumaier-compensated sum of partials[b][k] over blocks b, in block order.
-// The loads of 16 rows are issued before their additions (same additions in
-// the same order), so the loop waits on memory once per 16 rows.
-__global__ void reduce_partials_kernel(const double* __restrict__ partials, int nblocks,
-                                       int slots, double* __restrict__ out) {
-  constexpr int U = 16;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < slots; k += gridDim.x * blockDim.x) {
-    double s = 0, c = 0;
-    for (int b0 = 0; b0 < nblocks; b0 += U) {
-      double v[U];
-#pragma unroll
-      for (int u = 0; u < U; u++)
-        v[u] = b0 + u < nblocks ? partials[(long long)(b0 + u) * slots + k] : 0.0;
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        if (b0 + u >= nblocks) break;
-        const double t = s + v[u];
-        c += (fabs(s) >= fabs(v[u])) ? (s - t) + v[u] : (v[u] - t) + s;
-        s = t;
-      }
+__device__ __forceinline__ void neumaier(double& s, double& c, double v) {
+  const double t = s + v;
+  c += fabs(s) >= fabs(v) ? (s - t) + v : (v - t) + s;
+  s = t;
+}
+
+// out[k] = the sum of partials[b][k] over blocks b: one block per slot,
+// Neumaier-compensated sums per thread (rows t, t + 256, ...) and a fixed
+// tree over the threads.  (One thread per slot walking all rows took 0.18 ms
+// of a 0.9 ms objective pass.)
+constexpr int RP_T = 256;
+__global__ void __launch_bounds__(RP_T) reduce_partials_kernel(const double* __restrict__ partials,
+                                                               int nblocks, int slots,
+                                                               double* __restrict__ out) {
+  __shared__ double sh[RP_T], sc[RP_T];
+  const int k = blockIdx.x, t = threadIdx.x;
+  double s = 0, c = 0;
+  for (int b = t; b < nblocks; b += RP_T) neumaier(s, c, partials[(long long)b * slots + k]);
+  sh[t] = s;
+  sc[t] = c;
+  for (int w = RP_T / 2; w; w >>= 1) {
+    __syncthreads();
+    if (t < w) {
+      neumaier(s, c, sh[t + w]);
+      c += sc[t + w];
+      sh[t] = s;
+      sc[t] = c;
     }
-    out[k] = s + c;
   }
+  if (t == 0) out[k] = s + c;
 }
 
 // computeBottomBulkScalarGradientAP starts its overflow pass from zeroed
@@ -673,28 +837,38 @@ __global__ void bottom_bulk_fix_kernel(double* __restrict__ out, int nt, int nb)
 
 int tanh_slots(int nt, int nb) { return 8 + nt + nb; }
 
-int tanh_blocks() {
+// Voxels of one block: 32 while the blocks then number at most twice the
+// resident ones (16 warps per SM), 128 beyond, more where the partial rows
+// would outnumber 2^14.
+static long long tanh_per_block(long long n) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms * 4;
+  if (n <= 2ll * 32 * 16 * sms) return 32;
+  return std::max<long long>(128, (n / (1 << 14) + 32) / 32 * 32);
+}
+
+int tanh_blocks(long long n_voxels) {
+  const long long per = tanh_per_block(n_voxels);
+  return (int)((n_voxels + per - 1) / per);
 }
 
 cudaError_t launch_tanh_grad(const MapParams& m, const GridParams& g, const WeightGrid& wg,
                              const double* weights, int max_it, double alpha, double thr,
-                             bool pow_ref, double* field, double* partials, int nblocks,
-                             double* out, cudaStream_t s) {
+                             double* field, double* partials, double* out, cudaStream_t s) {
   const int slots = tanh_slots(m.nt, m.nb);
-  const size_t sh = sizeof(double) * (EN_T / 32) * slots;
-  if (pow_ref)
-    tanh_grad_kernel<true><<<nblocks, EN_T, sh, s>>>(m, g, wg, weights, max_it, alpha, thr, field,
-                                                     partials, slots);
+  const size_t sh = sizeof(double) * slots;
+  const long long n = (long long)g.X * g.Y * g.Z, per = tanh_per_block(n);
+  const int nblocks = tanh_blocks(n);
+  if (max_it == 1)
+    tanh_grad_kernel<true><<<nblocks, 32, sh, s>>>(m, g, wg, weights, max_it, alpha, thr, field,
+                                                   partials, slots, per);
   else
-    tanh_grad_kernel<false><<<nblocks, EN_T, sh, s>>>(m, g, wg, weights, max_it, alpha, thr,
-                                                      field, partials, slots);
+    tanh_grad_kernel<false><<<nblocks, 32, sh, s>>>(m, g, wg, weights, max_it, alpha, thr, field,
+                                                    partials, slots, per);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  reduce_partials_kernel<<<1, 256, 0, s>>>(partials, nblocks, slots, out);
+  reduce_partials_kernel<<<slots, RP_T, 0, s>>>(partials, nblocks, slots, out);
   bottom_bulk_fix_kernel<<<1, 1, 0, s>>>(out, m.nt, m.nb);
   return cudaGetLastError();
 }

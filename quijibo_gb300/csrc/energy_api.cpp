@@ -115,13 +115,13 @@ int qjg_tanh_score_grad(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, int3
   QJ_CUDA(ctx, cudaSetDevice(ctx->device));
   const qj::GridParams g = qj_grid_params(grid, 0, grid->res[2]);
   const qj::WeightGrid wg = qj_weight_grid(weight_grid);
-  const int nblocks = qj::tanh_blocks();
+  const int nblocks = qj::tanh_blocks((long long)g.X * g.Y * g.Z);
   const int slots = qj::tanh_slots(m->nt, m->nb);
   double* d_part = nullptr;
   QJ_CUDA(ctx, qj_malloc_async(ctx, &d_part, sizeof(double) * ((size_t)nblocks + 1) * slots, s));
   double* d_out = d_part + (size_t)nblocks * slots;
-  cudaError_t e = qj::launch_tanh_grad(*m, g, wg, d_weights, max_it, alpha, threshold, true,
-                                       d_field, d_part, nblocks, d_out, s);
+  cudaError_t e = qj::launch_tanh_grad(*m, g, wg, d_weights, max_it, alpha, threshold, d_field,
+                                       d_part, d_out, s);
   std::vector<double> out(slots);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(out.data(), d_out, sizeof(double) * slots, cudaMemcpyDeviceToHost, s);

@@ -94,28 +94,51 @@ __device__ __forceinline__ unsigned exp_field(double v) {
 // (a zero or huge base, an angle within 2^-8 of 0 or pi, exponents outside
 // [1/16, 512), |e log|q|| >= 512) the library's form.  Fields of 64^3 voxels,
 // 12 / 6 roots, real exponents: see field64_kernel.
-__device__ __forceinline__ Q qpow(const Q& q, double e) {
+// With LOG also what a derivative with respect to e takes: *l = log|q| and
+// *a = angle / |v| (log q = (*l, *a v)), and *amp = |q|^e.
+struct PowLog {
+  double l, a, amp;
+};
+static __device__ __noinline__ PowLog qpow_any_log(const Q q, double e) {
+  const double partial = add(add(mul(q.x, q.x), mul(q.y, q.y)), mul(q.z, q.z));
+  const double qm = __dsqrt_rn(add(partial, mul(q.w, q.w)));
+  const double vm = __dsqrt_rn(partial);
+  const double l = log(qm);
+  return PowLog{l, vm > 0.0 ? __ddiv_rn(acos(__ddiv_rn(q.w, qm)), vm) : 0.0, exp(mul(e, l))};
+}
+
+template <bool LOG = false>
+__device__ __forceinline__ Q qpow(const Q& q, double e, PowLog* pl = nullptr) {
   const double partial = add(add(mul(q.x, q.x), mul(q.y, q.y)), mul(q.z, q.z));
   const double n2 = add(partial, mul(q.w, q.w));
   // partial and n2 in [2^-200, 2^200) and positive, e in [1/16, 512)
   const bool in_range = exp_field(partial) - 823u < 400u && exp_field(n2) - 823u < 400u &&
                         exp_field(e) - 1019u < 13u;
-  if (!in_range) return qpow_any(q, e);
+  if (!in_range) {
+    if (LOG) *pl = qpow_any_log(q, e);
+    return qpow_any(q, e);
+  }
   const fx_roots rv = fx_sqrt_inv(partial), rq = fx_sqrt_inv(n2);
   fx_num w = fx_unpack(fabs(q.w));
   if ((exp_field(q.w) & 0x7ffu) < 600u) w.m = 0;  // below 2^-423: u = 0 to 2^-64
   int far = 0;
   const double th = fx_acos(w, rq.inv, rq.e, __double2hiint(q.w) < 0, &far);
-  const double x = mul(e, fx_log(rq.root));
+  const double l = fx_log(rq.root);
+  const double x = mul(e, l);
   const unsigned xe = exp_field(x) & 0x7ffu;
-  if (far || xe >= 1032u) return qpow_any(q, e);
-  const double scale = mul(mul(e, th), fx_pack62(rv.inv, -rv.e));
+  if (far || xe >= 1032u) {
+    if (LOG) *pl = qpow_any_log(q, e);
+    return qpow_any(q, e);
+  }
+  const double vminv = fx_pack62(rv.inv, -rv.e);
+  const double scale = mul(mul(e, th), vminv);
   const double m = mul(scale, rv.root);
   const double minv = fx_rcp(m);
   const double exps = xe < 964u ? 1.0 : fx_exp(x);
   double s, c;
   fx_sincos(m, &s, &c);
   const double scale2 = mul(mul(mul(scale, exps), minv), s);
+  if (LOG) *pl = PowLog{l, mul(th, vminv), exps};
   Q o;
   o.w = mul(exps, c);
   o.x = mul(scale2, q.x);

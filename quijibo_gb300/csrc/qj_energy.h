@@ -10,15 +10,15 @@ namespace qj {
 // A FIELD_3D weight grid for trilinear lookups (FIELD_3D.cpp:966-1029):
 // corner = center - lengths/2 + dx/2, inv = 1/dx.
 
-int tanh_blocks();
+// Blocks (rows of partials) of launch_tanh_grad on a grid of that many voxels.
+int tanh_blocks(long long n_voxels);
 // out[] of launch_tanh_grad: [d log s, d bottom exps, d top exps, d sigma_t,
 // d sigma_b, score, overflowed voxels, non-finite terms left out, scratch,
 // voxels with per-parameter terms]
 int tanh_slots(int nt, int nb);
 cudaError_t launch_tanh_grad(const MapParams& m, const GridParams& g, const WeightGrid& wg,
                              const double* weights, int max_it, double alpha, double thr,
-                             bool pow_ref, double* field, double* partials, int nblocks,
-                             double* out, cudaStream_t s);
+                             double* field, double* partials, double* out, cudaStream_t s);
 
 int sq_max_iterations();
 // Device scratch of one energy call (forward, or forward + gradient).

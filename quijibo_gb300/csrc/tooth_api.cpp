@@ -99,7 +99,7 @@ int qjg_tanh_fit(qjg_ctx* ctx, int32_t mode, qjg_map_state* state, const qjg_gri
   const int n = lay.n();
   const qj::GridParams g = qj_grid_params(grid, 0, grid->res[2]);
   const qj::WeightGrid wg = qj_weight_grid(weight_grid);
-  const int nblocks = qj::tanh_blocks();
+  const int nblocks = qj::tanh_blocks((long long)g.X * g.Y * g.Z);
   const int slots = qj::tanh_slots(nt, nb);
   double* d_part = nullptr;
   QJ_CUDA(ctx, qj_malloc_async(ctx, &d_part, sizeof(double) * ((size_t)nblocks + 1) * slots, s));
@@ -132,8 +132,8 @@ int qjg_tanh_fit(qjg_ctx* ctx, int32_t mode, qjg_map_state* state, const qjg_gri
       return 0;
     }
     // no field during the solve; d_field is filled once at the end
-    cudaError_t e = qj::launch_tanh_grad(m, g, wg, d_weights, max_it, alpha, threshold, true,
-                                         nullptr, d_part, nblocks, d_out, s);
+    cudaError_t e = qj::launch_tanh_grad(m, g, wg, d_weights, max_it, alpha, threshold, nullptr,
+                                         d_part, d_out, s);
     m_last = m;
     evaluated = true;
     if (e == cudaSuccess)
@@ -158,8 +158,8 @@ int qjg_tanh_fit(qjg_ctx* ctx, int32_t mode, qjg_map_state* state, const qjg_gri
   rc = qj::blmvm::minimize(n, x.data(), lo.data(), hi.data(), obj, mon, st, bs);
   if (!rc && d_field && evaluated) {
     // OPTIMIZE_3D::_fractal: the field of the last evaluation
-    cudaError_t e = qj::launch_tanh_grad(m_last, g, wg, d_weights, max_it, alpha, threshold, true,
-                                         d_field, d_part, nblocks, d_out, s);
+    cudaError_t e = qj::launch_tanh_grad(m_last, g, wg, d_weights, max_it, alpha, threshold, d_field,
+                                         d_part, d_out, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
       cuda_failed = 1;
