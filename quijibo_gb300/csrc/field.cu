@@ -450,9 +450,9 @@ __device__ __forceinline__ unsigned long long tile2(const MapParams& m, const Gr
   return __reduce_add_sync(0xffffffffu, (unsigned)(a.n + b.n));
 }
 
-// The unrolled forms (NT > 0) ask for 4 resident blocks per SM: ptxas then
-// keeps them at ~110 registers without spills, 3.7% faster at 16 / 8 roots
-// (the looped form is unchanged by it).
+// The forms with compiled-in counts (NT > 0) ask for 4 resident blocks per SM
+// (5: 512^3 at 16 / 8 roots 34.9 -> 35.9 ms; the looped form is unchanged by
+// it).
 template <bool DE, int NT = 0, int NB = 0>
 __global__ void __launch_bounds__(128, NT > 0 ? 4 : 0) field32x2_kernel(const __grid_constant__ MapParams m,
                                                         const GridParams g, const IterParams it,
@@ -744,10 +744,9 @@ cudaError_t launch_field32(const MapParams& m, const GridParams& g, const IterPa
   // the double-float head needs integer exponents and an error target
   const RefineLists rl = {list, keys, (refine && m.all_int && it.est_tol > 0.0) ? ff_list : nullptr};
   if (g_field32_pairs) {
-    // root counts of the benchmark maps compiled in: the precision form's
-    // 16 / 8 and the plain form's 8 / 0 fully unrolled (5% faster at 16 / 8),
-    // the large form's 48 / 24 two pairs per trip (8% faster; fully unrolled
-    // it ran 38% slower, instruction fetch); other maps read their counts
+    // root counts of the workloads' maps compiled in, two root pairs per trip
+    // (4% faster at 16 / 8 and at 48 / 24 roots than the kernel that reads
+    // its counts, which also ran 4% slower with two pairs per trip)
 #define QJ_F32X2(NT, NB)                                                                   \
   do {                                                                                     \
     const void* fn = want ? (const void*)field32x2_kernel<true, NT, NB>                   \
