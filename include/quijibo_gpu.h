@@ -167,7 +167,7 @@ typedef struct {
   int64_t n_tris;        /* triangles after the degenerate filter (or needed before it) */
   int64_t n_degenerate;  /* triangles dropped by the degenerate filter (edge < 1e-7) */
   int64_t n_unbracketed; /* edges whose end values do not bracket zero (the reference exits) */
-  int64_t map_evals;     /* FP64 map evaluations of the edge bisection */
+  int64_t map_evals;     /* FP64 map values the edge bisection used */
   int64_t map_evals_fp32;/* FP32 evaluations whose sign was trusted (precision form only) */
   int64_t map_evals_ff;  /* double-float evaluations that decided a point FP32 could not
                             (precision form, integer exponents) */

@@ -857,12 +857,42 @@ struct DegenEmit : DegenCount {
 
 // ------------------------------------------------------------ vertices
 
-// One vertex per listed edge: linear interpolation of the stored values
-// (computeEdgeInterpolations) or the bisection of midpointSearch on the map.
-// A bisection value log|q_N| - iso.  With HYBRID the FP32 orbit is tried
-// first and trusted when its value clears its error bound and the 1e-8 stop
-// test by a margin: then the FP64 value has the same sign and also fails the
-// stop test, so every decision of the search is the one FP64 would make.
+// One vertex per listed edge by linear interpolation of the stored values
+// (computeEdgeInterpolations).
+__global__ void __launch_bounds__(128) linear_kernel(const GridParams g,
+                                                     const uint32_t* __restrict__ list, long long n,
+                                                     long long id0, int c0,
+                                                     const double* __restrict__ src,
+                                                     double* __restrict__ verts, const McRun* run) {
+  if (run) {
+    if (run->overflow) return;
+    n = run->n_new;
+    id0 = run->nv;
+  }
+  using namespace q64;
+  const long long XY = (long long)g.X * g.Y;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x) {
+    const uint32_t e = list[k];
+    const int a = (int)(e & 3u);
+    const long long w = e >> 2;
+    const int z = c0 - 1 + (int)(w / XY);
+    const int r = (int)(w % XY);
+    const int x = r % g.X, y = r / g.X;
+    const int x1 = x + (a == 0), y1 = y + (a == 1), z1 = z + (a == 2);
+    double p0[3], p1[3];
+    cell_center(g, x, y, z, p0);
+    cell_center(g, x1, y1, z1, p1);
+    // TRIANGLE_MESH.cpp:2399-2410: p0 + (d0 / (d0 - d1)) * (p1 - p0)
+    const double d0 = src[(long long)(z - c0) * XY + r];
+    const double d1 = src[(long long)(z1 - c0) * XY + (long long)y1 * g.X + x1];
+    const double t = __ddiv_rn(d0, sub(d0, d1));
+    double* o = verts + 3 * (id0 + k);
+#pragma unroll
+    for (int c = 0; c < 3; c++) o[c] = add(p0[c], mul(t, sub(p1[c], p0[c])));
+  }
+}
+
 template <int POW_REF>
 __device__ __forceinline__ double value64(const MapParams& m, const GridParams& g,
                                           const IterParams& it, const double p[3], double iso,
@@ -874,133 +904,161 @@ __device__ __forceinline__ double value64(const MapParams& m, const GridParams& 
   return q64::sub(escape64<POW_REF, false>(m, it, p, g.slice, &ni, &dd), iso);
 }
 
-template <int POW_REF, bool HYBRID>
-__device__ __forceinline__ double bisect_value(const MapParams& m, const GridParams& g,
-                                               const IterParams& it, const double p[3], double iso,
-                                               unsigned long long* e32, unsigned long long* e64) {
-  if (HYBRID) {
-    float err;
-    const float f = escape32(m, it, p, g.slice, &err);
-    const float v = f - (float)iso;
-    if (fabsf(v) > 1.01f * err + 1e-8f + 1e-6f * fabsf((float)iso)) {
-      (*e32)++;
-      return (double)v;
-    }
-  }
-  return value64<POW_REF>(m, g, it, p, iso, e64);
-}
-
-template <bool BISECT, int POW_REF, bool HYBRID>
-__global__ void __launch_bounds__(128) vertex_kernel(const __grid_constant__ MapParams m,
-                                                     const GridParams g, const IterParams it,
-                                                     const uint32_t* __restrict__ list, long long n,
-                                                     long long id0, int c0,
-                                                     const double* __restrict__ src,
-                                                     double* __restrict__ verts, double iso,
-                                                     DevStats* st, const McRun* run) {
+// The bisection of midpointSearch (TRIANGLE_MESH.cpp:2060-2080, 2232-2271)
+// with every value in FP64.
+//
+// A vertex takes up to eight map evaluations one after the other, each a
+// chain of max_it applications, so few vertices leave the GPU waiting on that
+// chain (9.7 k vertices of a 48^3 mesh: two warps on a half of the SMs).
+// With at most `spec_max` edges a group of four lanes takes an edge: the two
+// ends at once, then per round the midpoint and the midpoints of both halves,
+// of which the midpoint's sign picks one: two levels per round.  More edges
+// fill the FP64 pipe with one lane each (the extra midpoint would cost a
+// third more).  `exact_ends`: the stored field is this map's FP64 value at
+// the grid points, so the ends need no evaluation.  The values used, and with
+// them every decision and vertex, are those of the one-by-one search; evals
+// counts those.  FP64 mesh of 48^3, 12 / 6 roots: 14.5 -> 9.3 ms a call.
+template <int POW_REF>
+__global__ void __launch_bounds__(32) bisect_kernel(const __grid_constant__ MapParams m,
+                                                    const GridParams g, const IterParams it,
+                                                    const uint32_t* __restrict__ list, long long n,
+                                                    long long id0, int c0,
+                                                    const double* __restrict__ src, int exact_ends,
+                                                    long long spec_max, double* __restrict__ verts,
+                                                    double iso, DevStats* st, const McRun* run) {
   if (run) {
     if (run->overflow) return;
     n = run->n_new;
     id0 = run->nv;
   }
+  using namespace q64;
   const long long XY = (long long)g.X * g.Y;
-  unsigned long long evals = 0, evals32 = 0, unbracketed = 0;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x) {
-    const uint32_t e = list[k];
-    const int a = (int)(e & 3u);
-    const long long w = e >> 2;
-    const int z = c0 - 1 + (int)(w / XY);
-    const int r = (int)(w % XY);
-    const int x = r % g.X, y = r / g.X;
-    const int x1 = x + (a == 0), y1 = y + (a == 1), z1 = z + (a == 2);
-    double p0[3], p1[3], out[3];
-    cell_center(g, x, y, z, p0);
-    cell_center(g, x1, y1, z1, p1);
-    using namespace q64;
-    if (!BISECT) {
-      // TRIANGLE_MESH.cpp:2399-2410: p0 + (d0 / (d0 - d1)) * (p1 - p0)
-      const double d0 = src[(long long)(z - c0) * XY + r];
-      const double d1 = src[(long long)(z1 - c0) * XY + (long long)y1 * g.X + x1];
-      const double t = __ddiv_rn(d0, sub(d0, d1));
+  const bool spec = n <= spec_max;
+  const int G = spec ? 4 : 1, lane = threadIdx.x, part = lane & (G - 1);
+  unsigned long long evals = 0, unbracketed = 0, applied = 0;
+  auto mid = [](const double* a, const double* b, double* o) {
 #pragma unroll
-      for (int c = 0; c < 3; c++) out[c] = add(p0[c], mul(t, sub(p1[c], p0[c])));
-    } else {
-      // nonlinearValue at both ends (TRIANGLE_MESH.cpp:2060-2067)
-      double f0 = bisect_value<POW_REF, HYBRID>(m, g, it, p0, iso, &evals32, &evals);
-      double f1 = bisect_value<POW_REF, HYBRID>(m, g, it, p1, iso, &evals32, &evals);
-      if (HYBRID && mul(f0, f1) >= 0.0) {
-        // the end values decide the whole search: confirm a failed bracket in FP64
-        f0 = value64<POW_REF>(m, g, it, p0, iso, &evals);
-        f1 = value64<POW_REF>(m, g, it, p1, iso, &evals);
-      }
-      double pv[3], nv[3], pval = f0, nval = f1;
-      bool bad = mul(f0, f1) >= 0.0;
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        pv[c] = p0[c];
-        nv[c] = p1[c];
-      }
-      if (f0 < 0) {
+    for (int c = 0; c < 3; c++) o[c] = mul(add(a[c], b[c]), 0.5);
+  };
+  for (long long base = (long long)blockIdx.x * (32 / G); base < n;
+       base += (long long)gridDim.x * (32 / G)) {
+    const long long k = base + lane / G;
+    double pv[3], nv[3], out[3], pval = 0, nval = 0;  // the positive and negative end
+    int stage = 3, rec = 0;                           // 0, 1: the ends; 2: bisection; 3: done
+    bool bad = false;
+    // the loop test of midpointSearch: where it stops, `out` is the vertex
+    auto settle = [&]() {
+      mid(pv, nv, out);
+      bad = mul(pval, nval) >= 0.0;
+      stage = bad || rec >= 6 ? 3 : 2;
+    };
+    // both end values known: positive end first
+    auto orient = [&]() {
+      if (pval < 0) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          pv[c] = p1[c];
-          nv[c] = p0[c];
+          const double t = pv[c];
+          pv[c] = nv[c];
+          nv[c] = t;
         }
-        pval = f1;
-        nval = f0;
+        const double t = pval;
+        pval = nval;
+        nval = t;
       }
-      // midpointSearch, TRIANGLE_MESH.cpp:2232-2271, as a loop
-      for (int rec = 0;; rec++) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) out[c] = mul(add(pv[c], nv[c]), 0.5);
-        if (mul(pval, nval) >= 0.0) {
-          bad = true;
-          break;
-        }
-        if (rec >= 6) break;
-        const double mv = bisect_value<POW_REF, HYBRID>(m, g, it, out, iso, &evals32, &evals);
-        if (fabs(mv) < 1e-8) break;
-        if (mv < 0) {
-#pragma unroll
-          for (int c = 0; c < 3; c++) nv[c] = out[c];
-          nval = mv;
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; c++) pv[c] = out[c];
-          pval = mv;
-        }
+      if (part == 0) evals += 2;
+      settle();
+    };
+    // one level with the value at `out`; whether the search goes on
+    auto level = [&](double v) {
+      if (part == 0) evals++;
+      if (fabs(v) < 1e-8) {
+        stage = 3;
+        return;
       }
+      double* end = v < 0 ? nv : pv;
+#pragma unroll
+      for (int c = 0; c < 3; c++) end[c] = out[c];
+      (v < 0 ? nval : pval) = v;
+      rec++;
+      settle();
+    };
+    if (k < n) {
+      const uint32_t e = list[k];
+      const int a = (int)(e & 3u);
+      const long long w = e >> 2;
+      const int z = c0 - 1 + (int)(w / XY);
+      const int r = (int)(w % XY);
+      const int x = r % g.X, y = r / g.X;
+      const int x1 = x + (a == 0), y1 = y + (a == 1), z1 = z + (a == 2);
+      cell_center(g, x, y, z, pv);
+      cell_center(g, x1, y1, z1, nv);
+      stage = 0;
+      if (exact_ends) {
+        pval = sub(src[(long long)(z - c0) * XY + r], iso);
+        nval = sub(src[(long long)(z1 - c0) * XY + (long long)y1 * g.X + x1], iso);
+        orient();
+      }
+    }
+    while (__any_sync(0xffffffffu, stage < 3)) {
+      double p[3] = {0, 0, 0}, v = 0;
+      bool has = stage < 3;
+      if (stage < 2) {
+        has = has && part < 2;
+        const bool first = spec ? part == 0 : stage == 0;
+#pragma unroll
+        for (int c = 0; c < 3; c++) p[c] = first ? pv[c] : nv[c];
+      } else if (part == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) p[c] = out[c];
+      } else {
+        has = has && part < 3 && rec < 5;
+        mid(part == 1 ? pv : out, part == 1 ? out : nv, p);
+      }
+      if (has) v = value64<POW_REF>(m, g, it, p, iso, &applied);
+      const double v0 = __shfl_sync(0xffffffffu, v, 0, G), v1 = __shfl_sync(0xffffffffu, v, 1 & (G - 1), G),
+                   v2 = __shfl_sync(0xffffffffu, v, 2 & (G - 1), G);
+      if (stage == 0) {
+        pval = v0;
+        nval = v1;
+        stage = 1;
+        if (spec) orient();
+      } else if (stage == 1) {
+        nval = v0;
+        orient();
+      } else if (stage == 2) {
+        level(v0);
+        if (spec && stage == 2) level(v0 < 0 ? v1 : v2);
+      }
+    }
+    if (k < n && part == 0) {
+      double* o = verts + 3 * (id0 + k);
+      o[0] = out[0];
+      o[1] = out[1];
+      o[2] = out[2];
       unbracketed += bad;
     }
-    double* o = verts + 3 * (id0 + k);
-    o[0] = out[0];
-    o[1] = out[1];
-    o[2] = out[2];
   }
-  if (BISECT) {
-    for (int o = 16; o; o >>= 1) {
-      evals += __shfl_xor_sync(0xffffffffu, evals, o);
-      evals32 += __shfl_xor_sync(0xffffffffu, evals32, o);
-      unbracketed += __shfl_xor_sync(0xffffffffu, unbracketed, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      if (evals) atomicAdd(&st->aux[1], evals);
-      if (unbracketed) atomicAdd(&st->aux[2], unbracketed);
-      if (evals32) atomicAdd(&st->aux[3], evals32);
-    }
+  for (int o = 16; o; o >>= 1) {
+    evals += __shfl_xor_sync(0xffffffffu, evals, o);
+    unbracketed += __shfl_xor_sync(0xffffffffu, unbracketed, o);
+  }
+  if (lane == 0) {
+    if (evals) atomicAdd(&st->aux[1], evals);
+    if (unbracketed) atomicAdd(&st->aux[2], unbracketed);
   }
 }
 
 // ------------------------------------------------- vertices, FP32 first
 
-// The FP32-first bisection with its FP64 evaluations taken out of line.  In
-// vertex_kernel<BISECT, *, HYBRID> a warp whose lane needs one FP64 map
-// evaluation waits for it at 1/64 of the FP32 rate while its other lanes
-// idle.  Here each edge carries its bisection state; an edge that needs an
-// FP64 value parks on a list, one kernel evaluates every parked point (a
-// warp of FP64 work), and the edges resume.  The decisions, and so the
-// vertices, are those of vertex_kernel.
+// The FP32-first bisection with its FP64 evaluations taken out of line.  A
+// value is first computed in FP32 and trusted when it clears its error bound
+// and the 1e-8 stop test by a margin: then the FP64 value has the same sign
+// and also fails the stop test, so every decision of the search is the one
+// FP64 would make.  In one kernel, a warp whose lane needs an FP64 map
+// evaluation would wait for it at 1/64 of the FP32 rate while its other lanes
+// idle.  So each edge carries its bisection state; an edge that needs an FP64
+// value parks on a list, one kernel evaluates every parked point (a warp of
+// FP64 work), and the edges resume.  The vertices are those of bisect_kernel.
 
 struct EdgeState {
   double a[3], b[3];  // stages 0-3: the edge's ends p0, p1; stage 4: positive, negative end
@@ -1545,29 +1603,48 @@ cudaError_t mesh_parked_finish(const MapParams& m, const GridParams& g, const It
                       : parked_finish<0>(m, g, it, verts, iso, st, sc, s);
 }
 
+// Edges up to which a group of lanes takes each: eight warps of whole edges
+// per SM, where one lane per edge begins to fill the FP64 pipe.
+static long long bisect_spec_max() { return (long long)sm_count() * 8 * 32; }
+
+static cudaError_t launch_bisect(int blocks, const MapParams& m, const GridParams& g,
+                                 const IterParams& it, int pow_mode, const uint32_t* list,
+                                 long long n, long long id0, int c0, const double* src,
+                                 bool exact_ends, long long spec_max, double* verts, double iso,
+                                 DevStats* st, const McRun* run, cudaStream_t s) {
+#define QJ_BK(P)                                                                               \
+  bisect_kernel<P><<<blocks, 32, 0, s>>>(m, g, it, list, n, id0, c0, src, exact_ends ? 1 : 0,  \
+                                         spec_max, verts, iso, st, run)
+  if (pow_mode == 2)
+    QJ_BK(2);
+  else if (pow_mode)
+    QJ_BK(1);
+  else
+    QJ_BK(0);
+#undef QJ_BK
+  return cudaGetLastError();
+}
+
 cudaError_t mesh_vertices(const MapParams& m, const GridParams& g, const IterParams& it,
-                          int edge_mode, int pow_mode, bool hybrid, const MeshWindow& w,
-                          long long n, long long id0, int c0, const double* src, double* verts,
-                          double iso, DevStats* st, const EdgeScratch* scratch, cudaStream_t s) {
+                          int edge_mode, int pow_mode, bool hybrid, bool exact_ends,
+                          const MeshWindow& w, long long n, long long id0, int c0,
+                          const double* src, double* verts, double iso, DevStats* st,
+                          const EdgeScratch* scratch, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (edge_mode != 0 && hybrid && scratch)
     return pow_mode == 2 ? parked_start<2>(m, g, it, w, n, id0, c0, verts, iso, st, *scratch, s)
            : pow_mode   ? parked_start<1>(m, g, it, w, n, id0, c0, verts, iso, st, *scratch, s)
                         : parked_start<0>(m, g, it, w, n, id0, c0, verts, iso, st, *scratch, s);
-  const int blocks = (int)std::min<long long>((n + 127) / 128, (long long)sm_count() * 32);
-#define QJ_VK(B, P, H) \
-  vertex_kernel<B, P, H><<<blocks, 128, 0, s>>>(m, g, it, w.list, n, id0, c0, src, verts, iso, st, \
-                                                nullptr)
-  if (edge_mode == 0)
-    QJ_VK(false, 0, false);
-  else if (pow_mode == 2)
-    hybrid ? QJ_VK(true, 2, true) : QJ_VK(true, 2, false);
-  else if (pow_mode)
-    hybrid ? QJ_VK(true, 1, true) : QJ_VK(true, 1, false);
-  else
-    hybrid ? QJ_VK(true, 0, true) : QJ_VK(true, 0, false);
-#undef QJ_VK
-  return cudaGetLastError();
+  if (edge_mode == 0) {
+    const int blocks = (int)std::min<long long>((n + 127) / 128, (long long)sm_count() * 32);
+    linear_kernel<<<blocks, 128, 0, s>>>(g, w.list, n, id0, c0, src, verts, nullptr);
+    return cudaGetLastError();
+  }
+  const long long spec_max = bisect_spec_max();
+  const long long warps = n <= spec_max ? (n + 7) / 8 : (n + 31) / 32;
+  return launch_bisect((int)std::min<long long>(warps, (long long)sm_count() * 64), m, g, it,
+                       pow_mode, w.list, n, id0, c0, src, exact_ends, spec_max, verts, iso, st,
+                       nullptr, s);
 }
 
 cudaError_t mesh_filter(const int32_t* tris, long long n, const double* verts, int32_t* out,
@@ -1655,9 +1732,10 @@ cudaError_t mesh_cube_scan_run(const MeshWindow& w, McCube* cubes, McRun* run,
 }
 
 cudaError_t mesh_vertices_run(const MapParams& m, const GridParams& g, const IterParams& it,
-                              int edge_mode, int pow_mode, bool hybrid, const MeshWindow& w,
-                              int c0, const double* src, double* verts, double iso, DevStats* st,
-                              const EdgeScratch* scratch, const McRun* run, cudaStream_t s) {
+                              int edge_mode, int pow_mode, bool hybrid, bool exact_ends,
+                              const MeshWindow& w, int c0, const double* src, double* verts,
+                              double iso, DevStats* st, const EdgeScratch* scratch,
+                              const McRun* run, cudaStream_t s) {
   const int blocks = sm_count() * 32;
   if (edge_mode != 0 && hybrid && scratch) {
 #define QJ_ES(P)                                                                              \
@@ -1673,18 +1751,12 @@ cudaError_t mesh_vertices_run(const MapParams& m, const GridParams& g, const Ite
 #undef QJ_ES
     return cudaGetLastError();
   }
-#define QJ_VK(B, P, H) \
-  vertex_kernel<B, P, H><<<blocks, 128, 0, s>>>(m, g, it, w.list, 0, 0, c0, src, verts, iso, st, run)
-  if (edge_mode == 0)
-    QJ_VK(false, 0, false);
-  else if (pow_mode == 2)
-    hybrid ? QJ_VK(true, 2, true) : QJ_VK(true, 2, false);
-  else if (pow_mode)
-    hybrid ? QJ_VK(true, 1, true) : QJ_VK(true, 1, false);
-  else
-    hybrid ? QJ_VK(true, 0, true) : QJ_VK(true, 0, false);
-#undef QJ_VK
-  return cudaGetLastError();
+  if (edge_mode == 0) {
+    linear_kernel<<<blocks, 128, 0, s>>>(g, w.list, 0, 0, c0, src, verts, run);
+    return cudaGetLastError();
+  }
+  return launch_bisect(2 * blocks, m, g, it, pow_mode, w.list, 0, 0, c0, src, exact_ends,
+                       bisect_spec_max(), verts, iso, st, run, s);
 }
 
 template <int POW_REF>

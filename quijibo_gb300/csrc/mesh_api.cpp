@@ -282,8 +282,12 @@ int mesh_core(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg_iter
       esc.list[0] = ctx->m_epark;
       esc.count = ctx->m_ecount;
     }
-    QJ_CUDA(ctx, qj::mesh_vertices(*m, g, it, edge_mode, pow_mode, hybrid, w, n_new, nv, c0, src,
-                                   ctx->m_verts, iso, ctx->d_mstats, parked ? &esc : nullptr, s));
+    // the slab's field is the bisection's own FP64 value at the grid points
+    // (the Lagrange bisection has a value of its own)
+    const bool exact_ends = streaming && !hybrid && iter->form == QJG_FORM_QUOTIENT;
+    QJ_CUDA(ctx, qj::mesh_vertices(*m, g, it, edge_mode, pow_mode, hybrid, exact_ends, w, n_new, nv,
+                                   c0, src, ctx->m_verts, iso, ctx->d_mstats,
+                                   parked ? &esc : nullptr, s));
     if (n_new) ctx->launches++;
     nv += n_new;
     QJ_CUDA(ctx, mark(3));
@@ -477,9 +481,10 @@ int mesh_core_async(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qj
     const long long u_split = last ? -1 : (long long)(L - 1) * Y * S;
     QJ_CUDA(ctx, qj::mesh_emit_run(w, src, P, Pv, c0, u_split, ctx->m_cubes[cur], ctx->m_run, s));
     QJ_CUDA(ctx, qj::mesh_cube_scan_run(w, ctx->m_cubes[cur], ctx->m_run, caps.cubes, s));
-    QJ_CUDA(ctx, qj::mesh_vertices_run(*m, g, it, QJG_EDGE_BISECT, pow_mode, hybrid, w, c0, src,
-                                       ctx->m_verts, iso, ctx->d_mstats, hybrid ? &esc : nullptr,
-                                       ctx->m_run, s));
+    const bool exact_ends = !hybrid && iter->form == QJG_FORM_QUOTIENT;
+    QJ_CUDA(ctx, qj::mesh_vertices_run(*m, g, it, QJG_EDGE_BISECT, pow_mode, hybrid, exact_ends, w,
+                                       c0, src, ctx->m_verts, iso, ctx->d_mstats,
+                                       hybrid ? &esc : nullptr, ctx->m_run, s));
     QJ_CUDA(ctx, qj::mesh_run_next(ctx->m_run, s));
     QJ_CUDA(ctx, qj::mesh_triangles_run(w, ctx->m_cubes[cur], last, c0 - 1, ctx->m_cubes[cur ^ 1],
                                         tris, tcap, ctx->m_run, s));

@@ -97,11 +97,13 @@ struct EdgeScratch {
 size_t mesh_edge_state_bytes();
 // Vertex placement (pow_mode as for launch_field64).  With hybrid bisection and a scratch, the edges that
 // need FP64 values are parked and their vertices written by
-// mesh_parked_finish after the last slab.
+// mesh_parked_finish after the last slab.  exact_ends: src holds the map's
+// own FP64 values (the plain form's field of this call).
 cudaError_t mesh_vertices(const MapParams& m, const GridParams& g, const IterParams& it,
-                          int edge_mode, int pow_mode, bool hybrid, const MeshWindow& w,
-                          long long n, long long id0, int c0, const double* src, double* verts,
-                          double iso, DevStats* st, const EdgeScratch* scratch, cudaStream_t s);
+                          int edge_mode, int pow_mode, bool hybrid, bool exact_ends,
+                          const MeshWindow& w, long long n, long long id0, int c0,
+                          const double* src, double* verts, double iso, DevStats* st,
+                          const EdgeScratch* scratch, cudaStream_t s);
 // Resolves every parked edge: rounds of one batched FP64 evaluation per
 // parked edge and a resumption (host reads of the list sizes in between).
 cudaError_t mesh_parked_finish(const MapParams& m, const GridParams& g, const IterParams& it,
@@ -127,9 +129,10 @@ cudaError_t mesh_emit_run(const MeshWindow& w, const double* src, int P, int Pv,
 cudaError_t mesh_cube_scan_run(const MeshWindow& w, McCube* cubes, McRun* run,
                                long long cap_cubes, cudaStream_t s);
 cudaError_t mesh_vertices_run(const MapParams& m, const GridParams& g, const IterParams& it,
-                              int edge_mode, int pow_mode, bool hybrid, const MeshWindow& w,
-                              int c0, const double* src, double* verts, double iso, DevStats* st,
-                              const EdgeScratch* scratch, const McRun* run, cudaStream_t s);
+                              int edge_mode, int pow_mode, bool hybrid, bool exact_ends,
+                              const MeshWindow& w, int c0, const double* src, double* verts,
+                              double iso, DevStats* st, const EdgeScratch* scratch,
+                              const McRun* run, cudaStream_t s);
 // the parked edges in a fixed number of rounds (8, the most any edge needs)
 cudaError_t mesh_parked_finish_fixed(const MapParams& m, const GridParams& g,
                                      const IterParams& it, int pow_mode, double* verts,
