@@ -310,9 +310,6 @@ struct OrbitLog {
   float2 step[2][ORBIT_WINDOW][128];  // {|q|^2, |grad log|R||^2} since the mark
 };
 
-__device__ __forceinline__ bool same_bits(float a, float b) {
-  return __float_as_int(a) == __float_as_int(b);
-}
 __device__ __forceinline__ bool same_bits(const q32::Q& a, const q32::Q& b) {
   return same_bits(a.w, b.w) && same_bits(a.x, b.x) && same_bits(a.y, b.y) && same_bits(a.z, b.z);
 }

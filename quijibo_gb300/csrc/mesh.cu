@@ -1086,7 +1086,7 @@ __device__ __forceinline__ void edge_point(const EdgeState& e, double p[3]) {
 template <int POW_REF>
 __device__ bool edge_advance(const MapParams& m, const GridParams& g, const IterParams& it,
                              EdgeState& e, double iso, double* vert, bool* bad,
-                             unsigned long long* e32) {
+                             unsigned long long* e32, PointLog<float>& log) {
   using namespace q64;
   for (;;) {
     double p[3];
@@ -1111,7 +1111,7 @@ __device__ bool edge_advance(const MapParams& m, const GridParams& g, const Iter
       return true;
     } else {
       float err;
-      const float f = escape32(m, it, p, g.slice, &err);
+      const float f = escape32(m, it, p, g.slice, &err, log);
       const float vf = f - (float)iso;
       if (!(fabsf(vf) > 1.01f * err + 1e-8f + 1e-6f * fabsf((float)iso))) return true;
       (*e32)++;
@@ -1214,7 +1214,7 @@ __device__ __forceinline__ void edge_counts(unsigned long long e32, unsigned lon
 
 // Starts every edge of the slab; edges that need FP64 go to `park`.
 template <int POW_REF>
-__global__ void __launch_bounds__(128) edge_start_kernel(const __grid_constant__ MapParams m,
+__global__ void __launch_bounds__(POINT_T) edge_start_kernel(const __grid_constant__ MapParams m,
                                                          const GridParams g, const IterParams it,
                                                          const uint32_t* __restrict__ list,
                                                          long long n, long long id0, int c0,
@@ -1228,6 +1228,7 @@ __global__ void __launch_bounds__(128) edge_start_kernel(const __grid_constant__
     n = run->n_new;
     id0 = run->nv;
   }
+  __shared__ PointLog<float> log;
   const long long XY = (long long)g.X * g.Y;
   unsigned long long e32 = 0, nbad = 0;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -1248,7 +1249,7 @@ __global__ void __launch_bounds__(128) edge_start_kernel(const __grid_constant__
       s.va = s.vb = s.pending = 0.0;
       s.stage = s.rec = s.flags = s.pad = 0;
       bool bad = false;
-      wait = edge_advance<POW_REF>(m, g, it, s, iso, verts + 3 * (id0 + k), &bad, &e32);
+      wait = edge_advance<POW_REF>(m, g, it, s, iso, verts + 3 * (id0 + k), &bad, &e32, log);
       nbad += bad;
       if (wait) es[id0 + k] = s;
     }
@@ -1261,7 +1262,7 @@ __global__ void __launch_bounds__(128) edge_start_kernel(const __grid_constant__
 // its tracked error bound decides what FP64 would (the sign, and in the
 // bisection whether |value| < 1e-8), that value stands in for FP64's; the
 // other edges, and the failed-bracket re-checks, go on to FP64 (`list64`).
-__global__ void __launch_bounds__(128) edge_ff_kernel(const __grid_constant__ MapParams m,
+__global__ void __launch_bounds__(POINT_T) edge_ff_kernel(const __grid_constant__ MapParams m,
                                                       const GridParams g, const IterParams it,
                                                       const uint32_t* __restrict__ park,
                                                       const unsigned long long* n_park,
@@ -1269,6 +1270,7 @@ __global__ void __launch_bounds__(128) edge_ff_kernel(const __grid_constant__ Ma
                                                       uint32_t* list64,
                                                       unsigned long long* n_list64,
                                                       DevStats* st) {
+  __shared__ PointLog<double> log;
   const unsigned long long n = *n_park;
   unsigned long long eff = 0;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -1285,7 +1287,7 @@ __global__ void __launch_bounds__(128) edge_ff_kernel(const __grid_constant__ Ma
         double p[3];
         edge_point(e, p);
         float err;
-        const double f = escape_ff(m, it, p, g.slice, &err);
+        const double f = escape_ff(m, it, p, g.slice, &err, log);
         const double v = f - iso;
         // FP64 rounding of f - iso and of the reference's own |q| on top
         const double eb = 1.01 * (double)err + 1e-15 * (fabs(f) + fabs(iso));
@@ -1330,7 +1332,7 @@ __global__ void __launch_bounds__(128) edge_fp64_kernel(const __grid_constant__ 
 
 // Resumes the parked edges; those that need FP64 again go to `next`.
 template <int POW_REF>
-__global__ void __launch_bounds__(128) edge_resume_kernel(const __grid_constant__ MapParams m,
+__global__ void __launch_bounds__(POINT_T) edge_resume_kernel(const __grid_constant__ MapParams m,
                                                           const GridParams g, const IterParams it,
                                                           const uint32_t* __restrict__ park,
                                                           const unsigned long long* n_park,
@@ -1339,6 +1341,7 @@ __global__ void __launch_bounds__(128) edge_resume_kernel(const __grid_constant_
                                                           uint32_t* next,
                                                           unsigned long long* n_next,
                                                           DevStats* st) {
+  __shared__ PointLog<float> log;
   const unsigned long long n = *n_park;
   unsigned long long e32 = 0, nbad = 0;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -1351,7 +1354,8 @@ __global__ void __launch_bounds__(128) edge_resume_kernel(const __grid_constant_
       k = park[j];
       EdgeState s = es[k];
       bool bad = false;
-      wait = edge_advance<POW_REF>(m, g, it, s, iso, verts + 3 * (long long)k, &bad, &e32);
+      wait = edge_advance<POW_REF>(m, g, it, s, iso, verts + 3 * (long long)k, &bad, &e32,
+                                   log);
       nbad += bad;
       if (wait) es[k] = s;
     }

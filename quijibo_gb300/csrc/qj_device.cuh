@@ -879,21 +879,45 @@ __device__ __forceinline__ q32x2::Q2 apply32x2(const MapParams& m, const q32x2::
   return out;
 }
 
+// A thread's marked iterate and the steps since, for the one-point loops
+// (kernels of POINT_T threads; shared memory): T float, or double for the
+// double-float loop, whose q has a high and a low part.
+constexpr int POINT_T = 128;
+template <class T>
+struct PointLog {
+  float4 mark[sizeof(T) / 4][POINT_T];
+  T m2[ORBIT_WINDOW][POINT_T];      // |q|^2 and |grad log|R||^2 of the steps
+  float gg[ORBIT_WINDOW][POINT_T];
+};
+
+__device__ __forceinline__ bool same_bits(float a, float b) {
+  return __float_as_int(a) == __float_as_int(b);
+}
+__device__ __forceinline__ bool same_bits(const float4& a, const float4& b) {
+  return same_bits(a.x, b.x) && same_bits(a.y, b.y) && same_bits(a.z, b.z) && same_bits(a.w, b.w);
+}
+
 // The FP32 escape loop at an arbitrary point: returns log|q_N| and, through
 // *err, the first-order estimate of its FP32 error (the relative error of
 // q_N carried by q32::propagate_err).  *err is infinite when FP32 cannot
 // follow the orbit (|q| below 1e-18, overflow) or an iterate lies within its
-// error of the escape radius.
+// error of the escape radius.  An orbit that comes back to an iterate bit for
+// bit is finished from its last period, as in the bulk pass (a 128^3 mesh at
+// 16 / 8 roots, whole call: 6.3 -> 4.4 ms).
 __device__ __forceinline__ float escape32(const MapParams& m, const IterParams& it,
-                                          const double p[3], double slice, float* err) {
+                                          const double p[3], double slice, float* err,
+                                          PointLog<float>& log) {
   using namespace q32;
+  const int tid = threadIdx.x;
   Q q = {(float)p[0], (float)p[1], (float)p[2], (float)slice};
   const float esc2 = (float)(it.escape * it.escape);
   float m2 = norm2(q), e = q32::EPS32;
-  int n = 0;
+  int n = 0, since = 0;
   bool bad = false, near = false;
+  log.mark[0][tid] = make_float4(q.w, q.x, q.y, q.z);
   while (m2 < esc2 && n < it.max_it) {
     float gg = 0.f;
+    const float4 before = make_float4(q.w, q.x, q.y, q.z);
     q = apply32<true>(m, q, &gg);
     near = near || q32::near_radius(m2, esc2, e);
     e = q32::propagate_err(e, gg, m2);
@@ -902,6 +926,27 @@ __device__ __forceinline__ float escape32(const MapParams& m, const IterParams& 
     if (m2 < 1e-36f) {
       bad = true;
       break;
+    }
+    if (!(m2 < esc2)) break;
+    log.m2[since][tid] = m2;
+    log.gg[since][tid] = gg;
+    since++;
+    const float4 now = make_float4(q.w, q.x, q.y, q.z);
+    const int period = same_bits(now, before) ? 1 : same_bits(now, log.mark[0][tid]) ? since : 0;
+    if (period) {
+      for (int j = since - period; n < it.max_it; n++) {
+        const float last = e;
+        near = near || q32::near_radius(m2, esc2, e);
+        e = q32::propagate_err(e, log.gg[j][tid], m2);
+        m2 = log.m2[j][tid];
+        if (period == 1 && same_bits(e, last)) n = it.max_it - 1;
+        j = j + 1 < since ? j + 1 : since - period;
+      }
+      break;
+    }
+    if (since >= mark_gap(n)) {
+      log.mark[0][tid] = now;
+      since = 0;
     }
   }
   // an iterate within FP32 error of the escape radius may stop the FP64

@@ -279,7 +279,8 @@ __device__ __forceinline__ qff::Q apply_ff(const MapParams& m, const qff::Q& q, 
 // radius (FP64 may stop at another iterate), |q| near the bottom of the FP32
 // exponent range the pairs live in, or a non-finite value.
 __device__ __forceinline__ double escape_ff(const MapParams& m, const IterParams& it,
-                                            const double p[3], double slice, float* err) {
+                                            const double p[3], double slice, float* err,
+                                            PointLog<double>& steps) {
   using namespace qff;
   Q q = {from_double(p[0]), from_double(p[1]), from_double(p[2]), from_double(slice)};
   const double esc2 = it.escape * it.escape;
@@ -289,7 +290,12 @@ __device__ __forceinline__ double escape_ff(const MapParams& m, const IterParams
   };
   double m2 = m2_of(q);
   float e = EPS_FF;
-  int n = 0;
+  int n = 0, since = 0;
+  const int tid = threadIdx.x;
+  auto high = [](const Q& v) { return make_float4(v.w.hi, v.x.hi, v.y.hi, v.z.hi); };
+  auto low = [](const Q& v) { return make_float4(v.w.lo, v.x.lo, v.y.lo, v.z.lo); };
+  steps.mark[0][tid] = high(q);
+  steps.mark[1][tid] = low(q);
   bool bad = false, near = false;
   // the escape test compares |q|^2 with esc^2 in FP64 here and |q| with esc
   // in the reference: a relative margin of 1e-14 covers the difference
@@ -298,6 +304,7 @@ __device__ __forceinline__ double escape_ff(const MapParams& m, const IterParams
   };
   while (m2 < esc2 && n < it.max_it) {
     float gg = 0.f;
+    const Q before = q;
     q = apply_ff<true>(m, q, &gg);
     near = near || near_esc(m2);
     e = q32::propagate_err_step(e, gg, (float)m2, ERR_STEP_FF);
@@ -306,6 +313,31 @@ __device__ __forceinline__ double escape_ff(const MapParams& m, const IterParams
     if (m2 < 1e-28) {
       bad = true;
       break;
+    }
+    if (!(m2 < esc2)) break;
+    // a repeating orbit is finished from its last period, as in escape32
+    steps.m2[since][tid] = m2;
+    steps.gg[since][tid] = gg;
+    since++;
+    const float4 hi = high(q), lo = low(q);
+    const int period = same_bits(hi, high(before)) && same_bits(lo, low(before)) ? 1
+                       : same_bits(hi, steps.mark[0][tid]) && same_bits(lo, steps.mark[1][tid]) ? since
+                                                                                            : 0;
+    if (period) {
+      for (int j = since - period; n < it.max_it; n++) {
+        const float last = e;
+        near = near || near_esc(m2);
+        e = q32::propagate_err_step(e, steps.gg[j][tid], (float)m2, ERR_STEP_FF);
+        m2 = steps.m2[j][tid];
+        if (period == 1 && same_bits(e, last)) n = it.max_it - 1;
+        j = j + 1 < since ? j + 1 : since - period;
+      }
+      break;
+    }
+    if (since >= mark_gap(n)) {
+      steps.mark[0][tid] = hi;
+      steps.mark[1][tid] = lo;
+      since = 0;
     }
   }
   bad = bad || near || (m2 >= esc2 && n < it.max_it && near_esc(m2));
