@@ -36,7 +36,8 @@ namespace qj {
 namespace {
 
 constexpr int SCAN_T = 256;              // threads per scan block
-constexpr int SCAN_V = 8;                // items per thread
+constexpr int SCAN_V = 2;                // items per thread (at 8, a 64-layer slab of 400 x
+                                         // 384 cells had 84 blocks for the 152 SMs)
 constexpr int SCAN_B = SCAN_T * SCAN_V;  // items per scan block
 
 // Edge id (1..12) -> lower-endpoint corner offset and axis (0=x, 1=y, 2=z),
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(SCAN_T) emit_kernel(Op op, long long n, const 
 // of one row of one plane, numbered in scan order (plane, row, segment)):
 // the sign words (every unit), and for units with activity (an edge with a
 // vertex or a cube with triangles) the packed counts of vertices and of
-// mixed cubes and the two activity words.  The unit counts start at zero.
+// mixed cubes.  The unit counts start at zero.
 // An exclusive scan of the counts gives every voxel's first vertex id and
 // every cube's place in the cube list in the reference's order (vertices by
 // (z, y, x, axis) of the edge's lower endpoint, cubes in scan order); the
@@ -235,8 +236,8 @@ struct McSlab {
   int gz0;            // global index of src plane 0
   long long XY;
   uint2* sign;        // [plane < P][Y][S]: sign words of every unit
-  uint2* bits;        // [Pv][Y][S]: activity words of units with activity
   uint32_t* ucount;   // [Pv][Y][S]: packed counts (zero where nothing is active)
+  int chunk;          // field planes of one classify task (the next plane is read too)
 };
 
 // Column validity of a segment starting at xb: x < X for even (vE) and odd
@@ -358,7 +359,6 @@ __device__ __forceinline__ void mc_classify_plane(const McSlab& c, int p, bool h
     }
   }
   uint32_t cnt_lane = 0;       // lane r: the packed counts of row r
-  uint2 bits_lane = {0u, 0u};  // lane r: the activity words of row r
 #pragma unroll
   for (int r = 0; r < MC_ROWS; r++) {
     const int y = y0 + r;
@@ -377,39 +377,54 @@ __device__ __forceinline__ void mc_classify_plane(const McSlab& c, int p, bool h
     if (!(actE | actO)) continue;  // uniform over the warp
     const int nv = __popc(xeE) + __popc(xeO) + __popc(yeE) + __popc(yeO) + __popc(zeE) + __popc(zeO);
     const int nc = __popc(mxE) + __popc(mxO);
-    if (lane == r) {
-      cnt_lane = unit_pack(nv, nc);
-      bits_lane = make_uint2(actE, actO);
-    }
+    if (lane == r) cnt_lane = unit_pack(nv, nc);
   }
   if (lane < MC_ROWS && cnt_lane) {
-    const long long u = ((long long)p * c.Y + y0 + lane) * c.S + seg;
-    c.ucount[u] = cnt_lane;
-    c.bits[u] = bits_lane;
+    c.ucount[((long long)p * c.Y + y0 + lane) * c.S + seg] = cnt_lane;
   }
 }
 
-// One warp per task (segment, row group).
+// The task of a warp: a segment, a row group and a range [q0, q1) of field
+// planes; plane q1 is read as the plane above where it exists.  A slab of
+// many rows is one range (no plane is read twice); a smaller one is cut into
+// ranges of at least 8 planes until the warps fill the SMs.
+struct McTask {
+  int seg, y0, q0, q1;
+};
+__device__ __forceinline__ bool mc_task(const McSlab& c, long long task, int planes, McTask* k) {
+  const int groups = (c.Y + MC_ROWS - 1) / MC_ROWS;
+  const long long per = (long long)groups * c.S;
+  k->q0 = (int)(task / per) * c.chunk;
+  if (k->q0 >= planes) return false;
+  const int r = (int)(task % per);
+  k->seg = r % c.S;
+  k->y0 = r / c.S * MC_ROWS;
+  k->q1 = min(k->q0 + c.chunk, planes);
+  return true;
+}
+
+// One warp per task.
 template <bool VEC>
 __global__ void __launch_bounds__(32 * MC_WARPS) mc_classify_kernel(const McSlab c) {
   const int lane = threadIdx.x & 31;
-  const long long task = (long long)blockIdx.x * MC_WARPS + (threadIdx.x >> 5);
-  const int groups = (c.Y + MC_ROWS - 1) / MC_ROWS;
-  if (task >= (long long)groups * c.S) return;  // the whole warp
-  const int seg = (int)(task % c.S);
-  const int y0 = (int)(task / c.S) * MC_ROWS;
-  const int xb = seg * MC_SEG;
+  const int planes = min(c.Pv + 1, c.P);  // planes read
+  McTask k;
+  if (!mc_task(c, (long long)blockIdx.x * MC_WARPS + (threadIdx.x >> 5), planes, &k)) return;
+  const int xb = k.seg * MC_SEG;
   const McCols v = mc_cols(c.X, xb);
   uint32_t lE[MC_ROWS + 1], lO[MC_ROWS + 1], lN;
-  plane_signs<VEC>(c.src, c.X, c.Y, y0, xb, lane, lE, lO, &lN);
-  for (int p = 0; p < c.Pv; p++) {
-    const bool hz = p + 1 < c.P;
+  plane_signs<VEC>(c.src + (long long)k.q0 * c.XY, c.X, c.Y, k.y0, xb, lane, lE, lO, &lN);
+  for (int p = k.q0; p < k.q1; p++) {
+    const bool hz = p + 1 < planes;
     uint32_t hE[MC_ROWS + 1], hO[MC_ROWS + 1], hN = 0;
 #pragma unroll
     for (int r = 0; r <= MC_ROWS; r++) hE[r] = hO[r] = 0u;
-    if (hz) plane_signs<VEC>(c.src + (long long)(p + 1) * c.XY, c.X, c.Y, y0, xb, lane, hE, hO, &hN);
-    store_signs(c, p, y0, seg, lane, lE, lO);
-    mc_classify_plane(c, p, hz, y0, seg, lane, v, lE, lO, lN, hE, hO, hN);
+    if (hz)
+      plane_signs<VEC>(c.src + (long long)(p + 1) * c.XY, c.X, c.Y, k.y0, xb, lane, hE, hO, &hN);
+    // (the window's top plane is stored for the emit pass even where it is
+    // not classified itself)
+    store_signs(c, p, k.y0, k.seg, lane, lE, lO);
+    if (p < c.Pv) mc_classify_plane(c, p, hz, k.y0, k.seg, lane, v, lE, lO, lN, hE, hO, hN);
 #pragma unroll
     for (int r = 0; r <= MC_ROWS; r++) {
       lE[r] = hE[r];
@@ -417,9 +432,6 @@ __global__ void __launch_bounds__(32 * MC_WARPS) mc_classify_kernel(const McSlab
     }
     lN = hN;
   }
-  // the window's top plane when it is not classified itself (the emit pass
-  // reads it as the plane above)
-  if (c.Pv < c.P) store_signs(c, c.Pv, y0, seg, lane, lE, lO);
 }
 
 // Form for fields whose rows are 16-byte aligned (X even): each lane copies
@@ -486,24 +498,23 @@ __device__ __forceinline__ void stage_signs(const unsigned char* stage, int lane
 __global__ void __launch_bounds__(32 * MC_WARPS) mc_classify_async_kernel(const McSlab c) {
   __shared__ __align__(16) unsigned char ring[MC_WARPS][MC_ASTAGES][MC_ASTAGE_BYTES];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long task = (long long)blockIdx.x * MC_WARPS + warp;
-  const int groups = (c.Y + MC_ROWS - 1) / MC_ROWS;
-  if (task >= (long long)groups * c.S) return;  // the whole warp
-  const int seg = (int)(task % c.S);
-  const int y0 = (int)(task / c.S) * MC_ROWS;
-  const int xb = seg * MC_SEG;
+  const int planes = min(c.Pv + 1, c.P);  // planes read
+  McTask k;
+  if (!mc_task(c, (long long)blockIdx.x * MC_WARPS + warp, planes, &k)) return;  // the whole warp
+  const int seg = k.seg, y0 = k.y0, xb = seg * MC_SEG;
   const McCols v = mc_cols(c.X, xb);
-  const int n_load = min(c.Pv + 1, c.P);  // planes read
+  const int end = min(k.q1 + 1, planes);  // with the plane above the range
 #pragma unroll
-  for (int q = 0; q < MC_ASTAGES; q++) async_plane(c, ring[warp][q], q, n_load, y0, xb, lane);
+  for (int q = 0; q < MC_ASTAGES; q++)
+    async_plane(c, ring[warp][q], k.q0 + q, end, y0, xb, lane);
   uint32_t lE[MC_ROWS + 1], lO[MC_ROWS + 1], lN = 0;
-  for (int q = 0; q < n_load; q++) {
-    unsigned char* st = ring[warp][q % MC_ASTAGES];
+  for (int q = k.q0; q < end; q++) {
+    unsigned char* st = ring[warp][(q - k.q0) % MC_ASTAGES];
     cp_async_wait_ahead();  // plane q has landed (this lane's copies)
     uint32_t hE[MC_ROWS + 1], hO[MC_ROWS + 1], hN;
     stage_signs(st, lane, hE, hO, &hN);
-    async_plane(c, st, q + MC_ASTAGES, n_load, y0, xb, lane);
-    if (q > 0) {  // voxel plane q - 1 between planes q - 1 and q
+    async_plane(c, st, q + MC_ASTAGES, end, y0, xb, lane);
+    if (q > k.q0) {  // voxel plane q - 1 between planes q - 1 and q
       store_signs(c, q - 1, y0, seg, lane, lE, lO);
       mc_classify_plane(c, q - 1, true, y0, seg, lane, v, lE, lO, lN, hE, hO, hN);
     }
@@ -514,14 +525,16 @@ __global__ void __launch_bounds__(32 * MC_WARPS) mc_classify_async_kernel(const 
     }
     lN = hN;
   }
-  // the last plane read: classified itself on the grid's last slab (no plane
-  // above), else stored as the window's top plane
-  store_signs(c, n_load - 1, y0, seg, lane, lE, lO);
-  if (c.Pv == n_load) {
-    uint32_t zE[MC_ROWS + 1], zO[MC_ROWS + 1];
+  if (k.q1 == planes) {
+    // the last plane read: classified itself on the grid's last slab (no
+    // plane above), else stored as the window's top plane
+    store_signs(c, planes - 1, y0, seg, lane, lE, lO);
+    if (c.Pv == planes) {
+      uint32_t zE[MC_ROWS + 1], zO[MC_ROWS + 1];
 #pragma unroll
-    for (int r = 0; r <= MC_ROWS; r++) zE[r] = zO[r] = 0u;
-    mc_classify_plane(c, n_load - 1, false, y0, seg, lane, v, lE, lO, lN, zE, zO, 0u);
+      for (int r = 0; r <= MC_ROWS; r++) zE[r] = zO[r] = 0u;
+      mc_classify_plane(c, planes - 1, false, y0, seg, lane, v, lE, lO, lN, zE, zO, 0u);
+    }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
@@ -665,11 +678,16 @@ __device__ __forceinline__ McRow load_row(const McSlab& c, int p, int y, int seg
   if (seg + 1 < c.S) r.next = c.sign[u + 1].x & 1u;
   return r;
 }
-__device__ __forceinline__ uint32_t bit_at(const McRow& r, int i) {
-  return i < 64 ? (uint32_t)(r.w >> i) & 1u : r.next;
-}
-
+// A scan block's threads first place their units, then eight lanes take each
+// unit with activity: they form its edge and cube words (the bit operations
+// of mc_classify_plane on words in x order), each lane ranks and writes the
+// voxels of its byte.  One thread per unit walked up to 64 voxels in series
+// (41 us per 64-layer slab of 400 x 384 cells, 40 us of 128 x 128); one warp
+// per unit left a scan block 32 units after one another (43 and 70 us); now 19 and 26.
 __global__ void __launch_bounds__(SCAN_T) mc_emit_kernel(const McEmit e, long long U) {
+  __shared__ int n_act;
+  __shared__ int act_unit[SCAN_B];
+  __shared__ uint2 act_base[SCAN_B];  // first vertex and cube, from the block's
   const McSlab& c = e.c;
   long long id0 = e.id0;
   McCube* cubes = e.cubes;
@@ -678,6 +696,7 @@ __global__ void __launch_bounds__(SCAN_T) mc_emit_kernel(const McEmit e, long lo
     id0 = e.run->nv;
     cubes += e.run->n_carry;
   }
+  if (threadIdx.x == 0) n_act = 0;
   const long long base = (long long)blockIdx.x * SCAN_B + (long long)threadIdx.x * SCAN_V;
   uint32_t cnt[SCAN_V];
   unsigned long long w = 0;
@@ -687,54 +706,81 @@ __global__ void __launch_bounds__(SCAN_T) mc_emit_kernel(const McEmit e, long lo
     w += unit_widen(cnt[k]);
   }
   unsigned long long total;
-  const unsigned long long ex = block_exclusive_scan(w, &total);
-  long long vp = e.bpre[2 * blockIdx.x] + (long long)(ex & 0xFFFFFFFFull);
-  long long cp = e.bpre[2 * blockIdx.x + 1] + (long long)(ex >> 32);
+  unsigned long long ex = block_exclusive_scan(w, &total);
+  const long long v0 = e.bpre[2 * blockIdx.x], q0 = e.bpre[2 * blockIdx.x + 1];
+#pragma unroll
   for (int k = 0; k < SCAN_V; k++) {
-    const long long u = base + k;
-    if (u == e.u_split) e.tot->split = cp;
-    if (!cnt[k]) continue;
+    if (base + k == e.u_split) e.tot->split = q0 + (long long)(ex >> 32);
+    if (cnt[k]) {
+      const int slot = atomicAdd(&n_act, 1);
+      act_unit[slot] = threadIdx.x * SCAN_V + k;
+      act_base[slot] = make_uint2((uint32_t)ex, (uint32_t)(ex >> 32));
+    }
+    ex += unit_widen(cnt[k]);
+  }
+  __syncthreads();
+  const int part = threadIdx.x & 7;
+  for (int t = threadIdx.x >> 3; t < (n_act + 3 & ~3); t += SCAN_T / 8) {  // whole warps
+    const bool on = t < n_act;
+    const long long u = on ? (long long)blockIdx.x * SCAN_B + act_unit[t] : 0;
     const int seg = (int)(u % c.S);
     const long long py = u / c.S;
     const int y = (int)(py % c.Y);
     const int p = (int)(py / c.Y);
-    const int gz = c.gz0 + p;
-    const int xb = seg * MC_SEG;
+    const int gz = c.gz0 + p, xb = seg * MC_SEG;
     const McRow A = load_row(c, p, y, seg), C = load_row(c, p, y + 1, seg);
     const McRow B = load_row(c, p + 1, y, seg), D = load_row(c, p + 1, y + 1, seg);
     const bool hy = y + 1 < c.Y, hz = p + 1 < c.P;
-    const long long r0 = (long long)y * c.X;
-    unsigned long long act = natural64(c.bits[u]);
-    while (act) {
-      const int i = __ffsll((long long)act) - 1;
-      act &= act - 1;
-      const int x = xb + i;
-      const bool hx = x + 1 < c.X;
-      const uint32_t a0 = bit_at(A, i), a1 = bit_at(A, i + 1);
-      const uint32_t b0 = bit_at(B, i), c0 = bit_at(C, i);
-      int m = (int)(hx & (a0 != a1)) | (int)(hy & (a0 != c0)) << 1 | (int)(hz & (a0 != b0)) << 2;
-      int f = 0;
-      if (hx && hy && hz)
-        f = (int)(a0 | b0 << 1 | c0 << 2 | bit_at(D, i) << 3 | a1 << 4 | bit_at(B, i + 1) << 5 |
-                  bit_at(C, i + 1) << 6 | bit_at(D, i + 1) << 7);
+    // words of the voxels' x + 1 neighbours; x < X and x + 1 < X
+    auto next = [](const McRow& r) { return r.w >> 1 | (unsigned long long)r.next << 63; };
+    const unsigned long long A1 = next(A), B1 = next(B), C1 = next(C), D1 = next(D);
+    const int nx = c.X - xb;
+    const unsigned long long in = nx >= 64 ? ~0ull : (1ull << nx) - 1ull;
+    const unsigned long long in1 = nx > 64 ? ~0ull : (1ull << (nx - 1)) - 1ull;
+    unsigned long long xe = (A.w ^ A1) & in1, ye = hy ? (A.w ^ C.w) & in : 0ull,
+                       ze = hz ? (A.w ^ B.w) & in : 0ull, mx = 0ull;
+    if (hy && hz) {
+      mx = (A.w | A1 | B.w | B1 | C.w | C1 | D.w | D1) & ~(A.w & A1 & B.w & B1 & C.w & C1 & D.w & D1) & in1;
       // the case-158 edges on the grid's boundary lines (mc_fix158_kernel)
-      if ((m & 1) && y == 0 && gz == 0 && f == 158) m &= ~1;
-      if (x == c.X - 1 && (m & 6)) {
-        if ((m & 2) && gz == 0 && cube_flag_src(c, x - 1, y, p) == 158) m &= ~2;
-        if ((m & 4) && y == 0 && cube_flag_src(c, x - 1, 0, p) == 158) m &= ~4;
-      }
-      const long long wv = (long long)(p + 1) * c.XY + r0 + x;
+      if (y == 0 && gz == 0) xe &= ~(~A.w & B.w & C.w & D.w & A1 & ~B1 & ~C1 & D1);
+    }
+    if (nx <= 64 && (y == 0 || gz == 0)) {
+      const unsigned long long last = 1ull << (nx - 1);
+      if (gz == 0 && (ye & last) && cube_flag_src(c, c.X - 2, y, p) == 158) ye &= ~last;
+      if (y == 0 && (ze & last) && cube_flag_src(c, c.X - 2, 0, p) == 158) ze &= ~last;
+    }
+    // this lane's byte, and the counts of the lower lanes' bytes
+    const unsigned bx = (unsigned)(xe >> 8 * part) & 255u, by = (unsigned)(ye >> 8 * part) & 255u,
+                   bz = (unsigned)(ze >> 8 * part) & 255u, bm = (unsigned)(mx >> 8 * part) & 255u;
+    const unsigned own = __popc(bx) + __popc(by) + __popc(bz) | __popc(bm) << 16;
+    unsigned sum = own;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const unsigned v = __shfl_up_sync(0xffffffffu, sum, o, 8);
+      if (part >= o) sum += v;
+    }
+    if (!on) continue;  // (no later shuffle in this trip; t is warp-uniform in count)
+    sum -= own;
+    long long vp = v0 + act_base[t].x + (sum & 0xffffu), cp = q0 + act_base[t].y + (sum >> 16);
+    for (unsigned act = bx | by | bz | bm; act; act &= act - 1) {
+      const int b = __ffs(act) - 1, i = 8 * part + b;
+      const int m = (int)(bx >> b & 1u) | (int)(by >> b & 1u) << 1 | (int)(bz >> b & 1u) << 2;
+      const uint32_t r = (uint32_t)((long long)y * c.X + xb + i);
       if (m) {
+        const long long wv = (long long)(p + 1) * c.XY + r;
         e.vbase[wv] = (int32_t)(id0 + vp);
         e.masks[wv] = (uint8_t)m;
 #pragma unroll
         for (int a = 0; a < 3; a++)
           if (m >> a & 1) e.list[vp++] = (uint32_t)(wv * 4 + a);
       }
-      if (f != 0 && f != 255) {
+      if (bm >> b & 1u) {
+        auto bit = [&](unsigned long long v) { return (uint32_t)(v >> i) & 1u; };
+        const uint32_t f = bit(A.w) | bit(B.w) << 1 | bit(C.w) << 2 | bit(D.w) << 3 | bit(A1) << 4 |
+                           bit(B1) << 5 | bit(C1) << 6 | bit(D1) << 7;
         McCube q;
-        q.r = (uint32_t)(r0 + x);
-        q.gzf = (uint32_t)gz | (uint32_t)f << 24;
+        q.r = r;
+        q.gzf = (uint32_t)gz | f << 24;
         q.tb = 0;
         cubes[cp++] = q;
       }
@@ -780,6 +826,10 @@ struct McTris {
 
 __global__ void __launch_bounds__(128) mc_tris_kernel(const McTris t, long long n_all) {
   __shared__ uint8_t cases[256][16];
+  __shared__ int4 edge[13];  // corner offset and axis (a divergent constant read is serial)
+  if (threadIdx.x < 13)
+    edge[threadIdx.x] = make_int4(c_edge_off[threadIdx.x][0], c_edge_off[threadIdx.x][1],
+                                  c_edge_off[threadIdx.x][2], c_edge_axis[threadIdx.x]);
   long long n_carry = t.n_carry;
   if (t.run) {
     if (t.run->overflow) return;
@@ -800,11 +850,9 @@ __global__ void __launch_bounds__(128) mc_tris_kernel(const McTris t, long long 
       if (k >= t.cap) continue;
 #pragma unroll
       for (int cc = 0; cc < 3; cc++) {
-        const int ed = cases[f][3 * tr + cc];
-        const long long v = (long long)(j + c_edge_off[ed][2]) * t.XY +
-                            (long long)(y + c_edge_off[ed][1]) * t.X + (x + c_edge_off[ed][0]);
-        const int a = c_edge_axis[ed];
-        t.tris[3 * k + cc] = t.vbase[v] + __popc(t.masks[v] & ((1 << a) - 1));
+        const int4 ed = edge[cases[f][3 * tr + cc]];
+        const long long v = (long long)(j + ed.z) * t.XY + (long long)(y + ed.y) * t.X + (x + ed.x);
+        t.tris[3 * k + cc] = t.vbase[v] + __popc(t.masks[v] & ((1 << ed.w) - 1));
       }
     }
   }
@@ -834,6 +882,29 @@ __device__ __forceinline__ double edge_len(const double* a, const double* b) {
   return __dsqrt_rn(add(add(mul(d0, d0), mul(d1, d1)), mul(d2, d2)));
 }
 
+// A double's leading 24 bits as a float, by integer operations (its size
+// within 2^-126 .. 2^127; 0 below, infinite beyond).
+__device__ __forceinline__ float leading24(double v) {
+  const int hi = __double2hiint(v), e = (hi >> 20 & 0x7ff) - 896;
+  if (e <= 0) return 0.0f;
+  if (e >= 255) return __int_as_float(0x7f800000);
+  return __int_as_float((hi & (int)0x80000000) | e << 23 | (hi & 0xfffff) << 3 |
+                        (int)((unsigned)__double2loint(v) >> 29));
+}
+// Whether a and b lie more than 1e-7 apart for certain: one coordinate
+// differs by more than ten times that and the truncation (2^-23 of each).
+// True of nearly every edge, where FP64 lengths kept the filter on the FP64
+// pipe (65 us for each of its two passes over 600 k triangles, 17 now).
+__device__ __forceinline__ bool far_apart(const double* a, const double* b) {
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const float x = leading24(a[c]), y = leading24(b[c]);
+    if (fabsf(x - y) > 1e-6f + 2.4e-7f * (fabsf(x) + fabsf(y)) && isfinite(x) && isfinite(y))
+      return true;
+  }
+  return false;
+}
+
 struct DegenCount {
   const int32_t* tris;
   const double* v;
@@ -841,6 +912,7 @@ struct DegenCount {
     const double* a = v + 3ll * tris[3 * t];
     const double* b = v + 3ll * tris[3 * t + 1];
     const double* c = v + 3ll * tris[3 * t + 2];
+    if (far_apart(a, b) && far_apart(a, c) && far_apart(b, c)) return 1;
     const double eps = 1e-7;
     return !(edge_len(a, b) < eps || edge_len(a, c) < eps || edge_len(b, c) < eps);
   }
@@ -1469,19 +1541,27 @@ static McSlab slab_of(const MeshWindow& w, const double* src, int P, int Pv, int
   c.gz0 = gz0;
   c.XY = (long long)w.X * w.Y;
   c.sign = reinterpret_cast<uint2*>(w.sign);
-  c.bits = reinterpret_cast<uint2*>(w.bits);
   c.ucount = w.ucount;
+  c.chunk = 0;
   return c;
 }
 
 cudaError_t mesh_classify(const MeshWindow& w, const double* src, int P, int Pv, int gz0,
                           cudaStream_t s) {
-  const McSlab c = slab_of(w, src, P, Pv, gz0);
+  McSlab c = slab_of(w, src, P, Pv, gz0);
   const long long U = mesh_units(w.X, w.Y, Pv);
   cudaError_t err;
   // units without activity keep these zero counts (the kernel stores the others)
   if ((err = cudaMemsetAsync(w.ucount, 0, (size_t)U * sizeof(uint32_t), s))) return err;
-  const long long tasks = (long long)c.S * ((c.Y + MC_ROWS - 1) / MC_ROWS);
+  // ranges of planes until there are 16 warps per SM, of at least 8 planes
+  // (a range reads one plane more): 64 layers of 400 x 384 cells 53 us as one
+  // range per warp, 32 us as 3 ranges
+  const long long per = (long long)c.S * ((c.Y + MC_ROWS - 1) / MC_ROWS);
+  const int planes = std::min(Pv + 1, P);
+  const long long ranges = std::min<long long>(std::max<long long>(1, 16ll * sm_count() / per),
+                                               std::max(1, planes / 8));
+  c.chunk = (int)((planes + ranges - 1) / ranges);
+  const long long tasks = per * ((planes + c.chunk - 1) / c.chunk);
   const unsigned blocks = (unsigned)((tasks + MC_WARPS - 1) / MC_WARPS);
   if ((w.X % 2 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0))
     mc_classify_async_kernel<<<blocks, 32 * MC_WARPS, 0, s>>>(c);

@@ -120,7 +120,6 @@ int mesh_core(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg_iter
   if ((rc = ensure(ctx, &ctx->m_masks, &ctx->m_masks_cap, wplanes)) ||
       (rc = ensure(ctx, &ctx->m_vbase, &ctx->m_vbase_cap, wplanes)) ||
       (rc = ensure(ctx, &ctx->m_sign, &ctx->m_sign_cap, (size_t)units * qj::MESH_UNIT_WORDS)) ||
-      (rc = ensure(ctx, &ctx->m_bits, &ctx->m_bits_cap, (size_t)units * qj::MESH_UNIT_WORDS)) ||
       (rc = ensure(ctx, &ctx->m_ucount, &ctx->m_ucount_cap, (size_t)units)) ||
       (rc = ensure(ctx, &ctx->m_tot, &ctx->m_tot_cap, (size_t)1)) ||
       (rc = ensure(ctx, &ctx->m_bsum, &ctx->m_bsum_cap,
@@ -139,7 +138,6 @@ int mesh_core(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg_iter
   w.vbase = ctx->m_vbase;
   w.list = ctx->m_list;
   w.bsum = ctx->m_bsum;
-  w.bits = ctx->m_bits;
   w.sign = ctx->m_sign;
   w.ucount = ctx->m_ucount;
   w.tot = ctx->m_tot;
@@ -441,7 +439,6 @@ int mesh_core_async(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qj
   w.vbase = ctx->m_vbase;
   w.list = ctx->m_list;
   w.bsum = ctx->m_bsum;
-  w.bits = ctx->m_bits;
   w.sign = ctx->m_sign;
   w.ucount = ctx->m_ucount;
   w.tot = ctx->m_tot;
@@ -546,7 +543,6 @@ int qjg_mesh_prepare(qjg_ctx* ctx, const qjg_grid* grid, int32_t slab_nz, int64_
   if ((rc = ensure(ctx, &ctx->m_masks, &ctx->m_masks_cap, wplanes)) ||
       (rc = ensure(ctx, &ctx->m_vbase, &ctx->m_vbase_cap, wplanes)) ||
       (rc = ensure(ctx, &ctx->m_sign, &ctx->m_sign_cap, (size_t)units * qj::MESH_UNIT_WORDS)) ||
-      (rc = ensure(ctx, &ctx->m_bits, &ctx->m_bits_cap, (size_t)units * qj::MESH_UNIT_WORDS)) ||
       (rc = ensure(ctx, &ctx->m_ucount, &ctx->m_ucount_cap, (size_t)units)) ||
       (rc = ensure(ctx, &ctx->m_tot, &ctx->m_tot_cap, (size_t)1)) ||
       (rc = ensure(ctx, &ctx->m_bsum, &ctx->m_bsum_cap, (size_t)caps.bsum)) ||

@@ -55,8 +55,6 @@ struct qjg_ctx {
   qj::DevStats* d_mstats = nullptr;
   double* m_field = nullptr;    // slab field window
   size_t m_field_cap = 0;
-  uint32_t* m_bits = nullptr;   // activity bits of the classified planes
-  size_t m_bits_cap = 0;
   uint32_t* m_sign = nullptr;   // sign words of the window's planes
   size_t m_sign_cap = 0;
   uint32_t* m_ucount = nullptr; // unit counts

@@ -45,8 +45,8 @@ struct McRun {
 
 // Scratch of one z-slab.  Window planes j <-> global plane c0 - 1 + j: edge
 // masks and vertex ids per window plane (plane c0 - 1 carried over from the
-// previous slab); per classified plane the activity bits, sparse voxel codes
-// and unit counts; the edge list of the slab's vertices; scan blocks.
+// previous slab); per classified plane the sign words and unit counts; the
+// edge list of the slab's vertices; scan blocks.
 struct MeshWindow {
   int X = 0, Y = 0;
   uint8_t* masks = nullptr;
@@ -54,7 +54,6 @@ struct MeshWindow {
   uint32_t* list = nullptr;
   long long* bsum = nullptr;  // 2 per scan block
   uint32_t* sign = nullptr;   // MESH_UNIT_WORDS per unit, every plane of the window
-  uint32_t* bits = nullptr;   // MESH_UNIT_WORDS per unit
   uint32_t* ucount = nullptr;
   McTotals* tot = nullptr;
 };
@@ -62,13 +61,12 @@ struct MeshWindow {
 long long mesh_scan_blocks(long long n);
 // classification units (row segments of one plane) of `planes` planes
 long long mesh_units(int X, int Y, int planes);
-// Words of activity bits per unit (64 voxels: even x, odd x).
+// Sign words per unit (64 voxels: even x, odd x).
 constexpr int MESH_UNIT_WORDS = 2;
 
 // Classify voxel planes [0, Pv) of src (P planes, global plane gz0 first;
 // Pv = P - 1, or P on the grid's last plane): sign words of every plane,
-// activity words and unit counts, their scan, the slab totals in w.tot (nv,
-// nc).
+// unit counts, their scan, the slab totals in w.tot (nv, nc).
 cudaError_t mesh_classify(const MeshWindow& w, const double* src, int P, int Pv, int gz0,
                           cudaStream_t s);
 // The slab's vertex ids, masks and edge list (window planes 1..Pv) and its
