@@ -15,6 +15,7 @@
 #include "../../include/quijibo_gpu.h"
 #include "../../include/quijibo_gpu_bench.h"
 #include "qj_ctx.h"
+#include "qj_fxmath.h"
 #include "qj_kernels.h"
 
 using qj::DevStats;
@@ -166,6 +167,12 @@ int qj_fill_map(MapParams* m, int n_top, const double* top_roots, const double* 
       m->rff[i][c][0] = m->r32[i][c];
       m->rff[i][c][1] = (float)(r[c] - (double)m->r32[i][c]);
     }
+    const fx_quat fq = fx_quat_of(r[0], r[1], r[2], r[3]);
+    m->rfx[i][0] = fq.w;
+    m->rfx[i][1] = fq.x;
+    m->rfx[i][2] = fq.y;
+    m->rfx[i][3] = fq.z;
+    m->efx[i] = fq.e;
     m->e64[i] = e;
     m->ep[i] = pw;
     m->e32[i] = (float)e;

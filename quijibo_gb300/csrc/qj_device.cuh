@@ -494,6 +494,47 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
   return r;
 }
 
+// The integer-power form's product of a side's terms in fixed point
+// (qj_fxmath.h), the product's exponent in *ex.  qx is q.  The FP64 pipe
+// issues 1/64 of what the integer pipe does: as fused FP64 products the
+// refine pass over a 128^3 grid whose inside needs it held that pipe at 80%
+// for 46 ms, as these it takes 11.7 ms (FP64 20%, ALU 62% busy); calls that
+// mesh 128^3 grids, one of three like that, went 24.5 -> 11.1 ms on average.
+// The product of 24 factors is off by 0.45 units of 2^-53 (rms), the fused
+// one by 3.8.
+template <bool DE>
+__device__ __forceinline__ q64::Q product_fx(const MapParams& m, const q64::Q& q,
+                                             const fx_quat& qx, int lo, int hi, double sign,
+                                             q64::Q& g, int* ex) {
+  using namespace q64;
+  fx_quat r;
+#pragma unroll 1
+  for (int i = lo; i < hi; i++) {
+    if (DE) {
+      // no reference counterpart: gradient of log|R| for the distance estimate
+      const Q d{sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
+                sub(q.z, m.r64[i][3])};
+      const double k = sign * m.e64[i] / norm2(d);
+      g.w += k * d.w;
+      g.x += k * d.x;
+      g.y += k * d.y;
+      g.z += k * d.z;
+    }
+    const fx_quat root{m.rfx[i][0], m.rfx[i][1], m.rfx[i][2], m.rfx[i][3], m.efx[i]};
+    fx_quat b = fx_qsub(qx, root);
+    if (fx_near(b, qx, root))  // rare: FP64's own difference keeps the low bits
+      b = fx_quat_of(sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
+                     sub(q.z, m.r64[i][3]));
+    const int e = m.ie[i];
+    fx_quat t = b;
+    if (e > 1) t = fx_qsq(b);
+    for (int k = 2; k < e; k++) t = fx_qmul(t, b);
+    r = i == lo ? t : fx_qmul(r, t);
+  }
+  *ex = r.e - 62;
+  return Q{(double)r.w, (double)r.x, (double)r.y, (double)r.z};
+}
+
 // RATIONAL_4D::evaluateLagrange (RATIONAL_4D.cpp:27-73): from 1, times top
 // term k then divided by bottom term k for the common k, then the longer
 // side's leftovers; without bottom roots the plain factored top.
@@ -526,6 +567,17 @@ __device__ __forceinline__ q64::Q apply64(const MapParams& m, const q64::Q& q, d
   Q out;
   if (lagrange) {
     out = lagrange64<POW_REF, DE>(m, q, g);
+  } else if (POW_REF == 0) {
+    int et, eb = 0;
+    const fx_quat qx = fx_quat_of(q.w, q.x, q.y, q.z);
+    const Q top = product_fx<DE>(m, q, qx, 0, m.nt, 1.0, g, &et);
+    out = top;
+    if (m.nb > 0) {
+      const Q bot = product_fx<DE>(m, q, qx, m.nt, m.nt + m.nb, -1.0, g, &eb);
+      out = fdiv(top, bot);
+    }
+    const int k = et - eb;
+    out = Q{fx_scale(out.w, k), fx_scale(out.x, k), fx_scale(out.y, k), fx_scale(out.z, k)};
   } else {
     const Q top = product64<POW_REF, DE>(m, q, 0, m.nt, 1.0, g);
     out = top;
@@ -559,7 +611,8 @@ __device__ __forceinline__ int mark_gap(int step) { return step < 12 ? 2 : ORBIT
 // no distance estimate where none is asked for, the FP64 part of whole
 // qjg_field calls went (2200 x 2200 x 4, 48 / 24 roots) 21.8 -> 11.4 ms,
 // (203 x 171 x 139, 23 / 11 roots) 5.2 -> 3.4 ms, (32^3, 12 / 4 roots) 1.02
-// -> 0.45 ms; a 128^3 mesh 151 -> 43 ms (three maps, one refined inside).
+// -> 0.45 ms; a 128^3 mesh 151 -> 43 ms (three maps, one refined inside;
+// 11.1 ms with product_fx).
 template <int POW_REF, bool DE>
 __device__ __forceinline__ double escape64(const MapParams& m, const IterParams& it,
                                            const double p[3], double slice, int* iters,
