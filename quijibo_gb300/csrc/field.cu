@@ -195,8 +195,14 @@ __device__ __forceinline__ int orbit_finish(const Orbit32& o, const IterParams& 
         DE && (o.near || (o.m2 >= esc2 && o.n < it.max_it && q32::near_radius(o.m2, esc2, o.err)));
     if (bad || near_escape || l2abs_d < l2band || fabsf(f) < it.field_tolf)
       route = TO_FP64;
-    else if (it.est_tolf > 0.f && !(o.err <= it.est_tolf * fabsf(f)))
-      route = (allow_ff && it.ff_head > 0) ? TO_FF : TO_FP64;
+    else if (it.est_tolf > 0.f && !(o.err <= it.est_tolf * fabsf(f))) {
+      // A re-run whose orbit outlasts the double-float head ends with an
+      // error of at least ERR_STEP and with f within 0.2 of this one: where
+      // that cannot pass either, the voxel goes to FP64 at once.
+      const bool hopeless = o.n > it.ff_head && o.err < 0.1f &&
+                            it.est_tolf * (fabsf(f) + 0.2f) < q32::ERR_STEP;
+      route = (allow_ff && it.ff_head > 0 && !hopeless) ? TO_FF : TO_FP64;
+    }
   }
   if (route == WRITTEN) {
     field[i] = (double)f;
