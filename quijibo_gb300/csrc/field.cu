@@ -9,7 +9,7 @@
 // Kernels:
 //   field64_kernel  -- the plain FP64 form: the reference's escape loop
 //                      (OPTIMIZE_3D.cpp:1317-1362) with QUATERNION::pow per
-//                      root term, reference-exact rounding.
+//                      root term, reference-exact rounding with QJG_LIBM_CR.
 //   field32_kernel  -- the FP32 bulk form: integer exponents by repeated
 //                      products, the distance estimate, and a refine list of
 //                      voxels that must be recomputed in FP64.

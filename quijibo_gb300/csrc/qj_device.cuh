@@ -470,8 +470,9 @@ __device__ __forceinline__ q64::Q term64(const MapParams& m, const q64::Q& q, in
   return POW_REF == 2 ? qpow_cr(d, m.e64[i]) : POW_REF ? qpow(d, m.e64[i]) : fpow(d, m.ie[i]);
 }
 
-// The product and the quotient of the form: reference order and rounding
-// for the polar powers, fused for the integer ones.
+// The FP64 chain's product and quotient (the Lagrange order, the correctly
+// rounded functions, maps out of product_fx's range): reference order and
+// rounding for the polar powers, fused for the integer ones.
 template <int POW_REF>
 __device__ __forceinline__ q64::Q times64(const q64::Q& a, const q64::Q& b) {
   return POW_REF ? q64::qmul(a, b) : q64::fmul(a, b);
@@ -494,42 +495,55 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
   return r;
 }
 
-// The integer-power form's product of a side's terms in fixed point
-// (qj_fxmath.h), the product's exponent in *ex.  qx is q.  The FP64 pipe
-// issues 1/64 of what the integer pipe does: as fused FP64 products the
-// refine pass over a 128^3 grid whose inside needs it held that pipe at 80%
-// for 46 ms, as these it takes 11.7 ms (FP64 20%, ALU 62% busy); calls that
-// mesh 128^3 grids, one of three like that, went 24.5 -> 11.1 ms on average.
-// The product of 24 factors is off by 0.45 units of 2^-53 (rms), the fused
-// one by 3.8.
-template <bool DE>
+// The product of a side's terms in fixed point (qj_fxmath.h), the product's
+// exponent in *ex; *odd where a term or a partial product leaves [2^-500,
+// 2^500], zero or not finite: there the FP64 chain's own overflow, underflow
+// and NaN count.  qx is q.  The FP64 pipe issues 1/64 of what the integer
+// pipe does: as fused FP64 products the refine pass over a 128^3 grid whose
+// inside needs it held that pipe at 80% for 46 ms, as these it takes 11.7 ms
+// (FP64 20%, ALU 62% busy); calls that mesh 128^3 grids, one of three like
+// that, went 24.5 -> 11.1 ms on average.  The polar powers' products, 28 of
+// a term's 52 FP64 instructions in the reference's order: plain FP64 field
+// 64^3 6.7 -> 5.3 ms, FP64 mesh 48^3 9.2 -> 6.9 ms (12 / 6 roots).  The
+// product of 24 factors is off by 0.45 units of 2^-53 (rms), the fused one
+// by 3.8.
+template <int POW_REF, bool DE>
 __device__ __forceinline__ q64::Q product_fx(const MapParams& m, const q64::Q& q,
                                              const fx_quat& qx, int lo, int hi, double sign,
-                                             q64::Q& g, int* ex) {
+                                             q64::Q& g, int* ex, bool* odd) {
   using namespace q64;
   fx_quat r;
 #pragma unroll 1
   for (int i = lo; i < hi; i++) {
+    Q d;
+    if (DE || POW_REF)
+      d = Q{sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
+            sub(q.z, m.r64[i][3])};
     if (DE) {
       // no reference counterpart: gradient of log|R| for the distance estimate
-      const Q d{sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
-                sub(q.z, m.r64[i][3])};
       const double k = sign * m.e64[i] / norm2(d);
       g.w += k * d.w;
       g.x += k * d.x;
       g.y += k * d.y;
       g.z += k * d.z;
     }
-    const fx_quat root{m.rfx[i][0], m.rfx[i][1], m.rfx[i][2], m.rfx[i][3], m.efx[i]};
-    fx_quat b = fx_qsub(qx, root);
-    if (fx_near(b, qx, root))  // rare: FP64's own difference keeps the low bits
-      b = fx_quat_of(sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
-                     sub(q.z, m.r64[i][3]));
-    const int e = m.ie[i];
-    fx_quat t = b;
-    if (e > 1) t = fx_qsq(b);
-    for (int k = 2; k < e; k++) t = fx_qmul(t, b);
+    fx_quat t;
+    if (POW_REF) {
+      const Q p = qpow(d, m.e64[i]);
+      t = fx_quat_of(p.w, p.x, p.y, p.z);
+    } else {
+      const fx_quat root{m.rfx[i][0], m.rfx[i][1], m.rfx[i][2], m.rfx[i][3], m.efx[i]};
+      fx_quat b = fx_qsub(qx, root);
+      if (fx_near(b, qx, root))  // rare: FP64's own difference keeps the low bits
+        b = fx_quat_of(sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
+                       sub(q.z, m.r64[i][3]));
+      const int e = m.ie[i];
+      t = b;
+      if (e > 1) t = fx_qsq(b);
+      for (int k = 2; k < e; k++) t = fx_qmul(t, b);
+    }
     r = i == lo ? t : fx_qmul(r, t);
+    *odd |= (unsigned)(t.e + 500) > 1000u || (unsigned)(r.e + 500) > 1000u;
   }
   *ex = r.e - 62;
   return Q{(double)r.w, (double)r.x, (double)r.y, (double)r.z};
@@ -557,7 +571,9 @@ __device__ __forceinline__ q64::Q lagrange64(const MapParams& m, const q64::Q& q
 }
 
 // One application of the map in reference order (OPTIMIZE_3D.cpp:1331-1350),
-// plus |grad log|R|| for the distance estimate when DE is set.
+// plus |grad log|R|| for the distance estimate when DE is set; the products
+// in fixed point, with the correctly rounded functions (POW_REF = 2) rounded
+// as the reference's.
 // With `lagrange`, the map in the Lagrange order (TRIANGLE_MESH.cpp:281-322).
 template <int POW_REF, bool DE>
 __device__ __forceinline__ q64::Q apply64(const MapParams& m, const q64::Q& q, double* gnorm,
@@ -567,23 +583,23 @@ __device__ __forceinline__ q64::Q apply64(const MapParams& m, const q64::Q& q, d
   Q out;
   if (lagrange) {
     out = lagrange64<POW_REF, DE>(m, q, g);
-  } else if (POW_REF == 0) {
-    int et, eb = 0;
-    const fx_quat qx = fx_quat_of(q.w, q.x, q.y, q.z);
-    const Q top = product_fx<DE>(m, q, qx, 0, m.nt, 1.0, g, &et);
-    out = top;
-    if (m.nb > 0) {
-      const Q bot = product_fx<DE>(m, q, qx, m.nt, m.nt + m.nb, -1.0, g, &eb);
-      out = fdiv(top, bot);
-    }
-    const int k = et - eb;
-    out = Q{fx_scale(out.w, k), fx_scale(out.x, k), fx_scale(out.y, k), fx_scale(out.z, k)};
   } else {
-    const Q top = product64<POW_REF, DE>(m, q, 0, m.nt, 1.0, g);
-    out = top;
-    if (m.nb > 0) {
-      const Q bot = product64<POW_REF, DE>(m, q, m.nt, m.nt + m.nb, -1.0, g);
-      out = over64<POW_REF>(top, bot);
+    bool odd = POW_REF == 2;
+    if (POW_REF != 2) {
+      int et, eb = 0;
+      fx_quat qx;
+      if (POW_REF == 0) qx = fx_quat_of(q.w, q.x, q.y, q.z);
+      out = product_fx<POW_REF, DE>(m, q, qx, 0, m.nt, 1.0, g, &et, &odd);
+      if (m.nb > 0)
+        out = fdiv(out, product_fx<POW_REF, DE>(m, q, qx, m.nt, m.nt + m.nb, -1.0, g, &eb, &odd));
+      const int k = et - eb;
+      out = Q{fx_scale(out.w, k), fx_scale(out.x, k), fx_scale(out.y, k), fx_scale(out.z, k)};
+    }
+    if (odd) {
+      g = Q{0.0, 0.0, 0.0, 0.0};
+      out = product64<POW_REF, DE>(m, q, 0, m.nt, 1.0, g);
+      if (m.nb > 0)
+        out = over64<POW_REF>(out, product64<POW_REF, DE>(m, q, m.nt, m.nt + m.nb, -1.0, g));
     }
   }
   out.w = mul(out.w, m.scale);
