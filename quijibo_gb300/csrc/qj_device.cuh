@@ -471,7 +471,7 @@ __device__ __forceinline__ q64::Q term64(const MapParams& m, const q64::Q& q, in
 }
 
 // The FP64 chain's product and quotient (the Lagrange order, the correctly
-// rounded functions, maps out of product_fx's range): reference order and
+// rounded functions, maps out of quotient_fx's range): reference order and
 // rounding for the polar powers, fused for the integer ones.
 template <int POW_REF>
 __device__ __forceinline__ q64::Q times64(const q64::Q& a, const q64::Q& b) {
@@ -495,33 +495,35 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
   return r;
 }
 
-// The product of a side's terms in fixed point (qj_fxmath.h), the product's
-// exponent in *ex; *odd where a term or a partial product leaves [2^-500,
+// The quotient of the sides' products, the products in fixed point
+// (qj_fxmath.h); *odd where a term or a partial product leaves [2^-500,
 // 2^500], zero or not finite: there the FP64 chain's own overflow, underflow
-// and NaN count.  qx is q.  The FP64 pipe issues 1/64 of what the integer
+// and NaN count.  The FP64 pipe issues 1/64 of what the integer
 // pipe does: as fused FP64 products the refine pass over a 128^3 grid whose
 // inside needs it held that pipe at 80% for 46 ms, as these it takes 11.7 ms
 // (FP64 20%, ALU 62% busy); calls that mesh 128^3 grids, one of three like
 // that, went 24.5 -> 11.1 ms on average.  The polar powers' products, 28 of
 // a term's 52 FP64 instructions in the reference's order: plain FP64 field
-// 64^3 6.7 -> 5.3 ms, FP64 mesh 48^3 9.2 -> 6.9 ms (12 / 6 roots).  The
-// product of 24 factors is off by 0.45 units of 2^-53 (rms), the fused one
-// by 3.8.
+// 64^3 6.7 -> 4.6 ms, FP64 mesh 48^3 9.2 -> 6.1 ms (12 / 6 roots; 5.3 and
+// 6.9 ms with a loop for each side and the FP64 chain expanded in place: the
+// code has to stay small for instruction fetch).  The product of 24 factors
+// is off by 0.45 units of 2^-53 (rms), the fused one by 3.8.
 template <int POW_REF, bool DE>
-__device__ __forceinline__ q64::Q product_fx(const MapParams& m, const q64::Q& q,
-                                             const fx_quat& qx, int lo, int hi, double sign,
-                                             q64::Q& g, int* ex, bool* odd) {
+__device__ __forceinline__ q64::Q quotient_fx(const MapParams& m, const q64::Q& q, q64::Q& g,
+                                              bool* odd) {
   using namespace q64;
-  fx_quat r;
+  fx_quat qx, r, top;
+  if (POW_REF == 0) qx = fx_quat_of(q.w, q.x, q.y, q.z);
+  const int nt = m.nt, n = nt + m.nb;
 #pragma unroll 1
-  for (int i = lo; i < hi; i++) {
+  for (int i = 0; i < n; i++) {
     Q d;
     if (DE || POW_REF)
       d = Q{sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
             sub(q.z, m.r64[i][3])};
     if (DE) {
       // no reference counterpart: gradient of log|R| for the distance estimate
-      const double k = sign * m.e64[i] / norm2(d);
+      const double k = (i < nt ? m.e64[i] : -m.e64[i]) / norm2(d);
       g.w += k * d.w;
       g.x += k * d.x;
       g.y += k * d.y;
@@ -542,11 +544,31 @@ __device__ __forceinline__ q64::Q product_fx(const MapParams& m, const q64::Q& q
       if (e > 1) t = fx_qsq(b);
       for (int k = 2; k < e; k++) t = fx_qmul(t, b);
     }
-    r = i == lo ? t : fx_qmul(r, t);
+    if (i == nt) top = r;
+    r = i == 0 || i == nt ? t : fx_qmul(r, t);
     *odd |= (unsigned)(t.e + 500) > 1000u || (unsigned)(r.e + 500) > 1000u;
   }
-  *ex = r.e - 62;
-  return Q{(double)r.w, (double)r.x, (double)r.y, (double)r.z};
+  Q out{(double)r.w, (double)r.x, (double)r.y, (double)r.z};
+  int k = r.e - 62;
+  if (n > nt) {
+    out = fdiv(Q{(double)top.w, (double)top.x, (double)top.y, (double)top.z}, out);
+    k = top.e - r.e;
+  }
+  return Q{fx_scale(out.w, k), fx_scale(out.x, k), fx_scale(out.y, k), fx_scale(out.z, k)};
+}
+
+// The same by the FP64 chain.
+template <int POW_REF, bool DE>
+__device__ __forceinline__ q64::Q quotient64(const MapParams& m, const q64::Q& q, q64::Q& g) {
+  g = q64::Q{0.0, 0.0, 0.0, 0.0};
+  const q64::Q top = product64<POW_REF, DE>(m, q, 0, m.nt, 1.0, g);
+  if (m.nb == 0) return top;
+  return over64<POW_REF>(top, product64<POW_REF, DE>(m, q, m.nt, m.nt + m.nb, -1.0, g));
+}
+template <int POW_REF, bool DE>
+static __device__ __noinline__ q64::Q quotient64_far(const MapParams& m, const q64::Q q,
+                                                     q64::Q* g) {
+  return quotient64<POW_REF, DE>(m, q, *g);
 }
 
 // RATIONAL_4D::evaluateLagrange (RATIONAL_4D.cpp:27-73): from 1, times top
@@ -583,23 +605,15 @@ __device__ __forceinline__ q64::Q apply64(const MapParams& m, const q64::Q& q, d
   Q out;
   if (lagrange) {
     out = lagrange64<POW_REF, DE>(m, q, g);
+  } else if (POW_REF == 2) {
+    out = quotient64<POW_REF, DE>(m, q, g);
   } else {
-    bool odd = POW_REF == 2;
-    if (POW_REF != 2) {
-      int et, eb = 0;
-      fx_quat qx;
-      if (POW_REF == 0) qx = fx_quat_of(q.w, q.x, q.y, q.z);
-      out = product_fx<POW_REF, DE>(m, q, qx, 0, m.nt, 1.0, g, &et, &odd);
-      if (m.nb > 0)
-        out = fdiv(out, product_fx<POW_REF, DE>(m, q, qx, m.nt, m.nt + m.nb, -1.0, g, &eb, &odd));
-      const int k = et - eb;
-      out = Q{fx_scale(out.w, k), fx_scale(out.x, k), fx_scale(out.y, k), fx_scale(out.z, k)};
-    }
+    bool odd = false;
+    out = quotient_fx<POW_REF, DE>(m, q, g, &odd);
     if (odd) {
-      g = Q{0.0, 0.0, 0.0, 0.0};
-      out = product64<POW_REF, DE>(m, q, 0, m.nt, 1.0, g);
-      if (m.nb > 0)
-        out = over64<POW_REF>(out, product64<POW_REF, DE>(m, q, m.nt, m.nt + m.nb, -1.0, g));
+      Q h;
+      out = quotient64_far<POW_REF, DE>(m, q, &h);
+      g = h;
     }
   }
   out.w = mul(out.w, m.scale);
@@ -628,7 +642,7 @@ __device__ __forceinline__ int mark_gap(int step) { return step < 12 ? 2 : ORBIT
 // qjg_field calls went (2200 x 2200 x 4, 48 / 24 roots) 21.8 -> 11.4 ms,
 // (203 x 171 x 139, 23 / 11 roots) 5.2 -> 3.4 ms, (32^3, 12 / 4 roots) 1.02
 // -> 0.45 ms; a 128^3 mesh 151 -> 43 ms (three maps, one refined inside;
-// 11.1 ms with product_fx).
+// 11.1 ms with quotient_fx).
 template <int POW_REF, bool DE>
 __device__ __forceinline__ double escape64(const MapParams& m, const IterParams& it,
                                            const double p[3], double slice, int* iters,
