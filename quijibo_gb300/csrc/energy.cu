@@ -2601,6 +2601,16 @@ __global__ void __launch_bounds__(32 * SQR_W) sq_reduce_item_kernel(
 std::atomic<int> g_sq_pairs{0};
 // Forward blocks per SM (qjg_set_energy_forward_blocks): 0 the rule in
 // sq_launch, else that many (capped by residency), for sweeps.
+// The forward grid's blocks per SM: three, more where a lane would get over
+// four samples.  A warp's lanes stay busy only while there are samples to
+// refill them, so more lanes pay only where nearly every orbit settles early
+// (us of an energy + gradient call at 3 / 4 / 5 / 8 blocks per SM, 200k
+// samples, 64/16 roots: 421 / 383 / 381 / 380; ms of a 50-step
+// L-BFGS fit of them, whose orbits spread more: 86 / 92 / 103 / 134).
+static long long sq_fwd_want(long long n, int sms) {
+  const long long lanes_per_sm = (long long)sms * SQF_T;
+  return std::max<long long>(3, ((n + 3) / 4 + lanes_per_sm - 1) / lanes_per_sm);
+}
 std::atomic<int> g_sq_fwd_blocks{0};
 
 // FP32 adjoint choice (qjg_set_energy_adjoint_roots): the roots of a step
@@ -2703,18 +2713,8 @@ cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const dou
   else
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sq_fwd_kernel<T, false>, SQF_T, sh_roots);
   if (e != cudaSuccess) return e;
-  // Blocks per SM: in FP32 as many as stay resident.  With the settled
-  // orbits cut short a sample takes about 4 map applications and the longest
-  // lanes are those few samples that do not settle, so more lanes only fill
-  // issue slots (energy + gradient call, us, at 3 / 4 / 5 / all blocks per
-  // SM: 200k samples, 64/16 roots 421 / 383 / 381 / 380; 100k, 32/16 roots
-  // 256 / 266 / 230 / 248; 50k and fewer samples within 1%).  FP64 (bound by
-  // the FP64 pipe) keeps about four samples per lane.
-  const long long lanes_per_sm = (long long)sms * SQF_T;
   const int fixed = g_sq_fwd_blocks.load(std::memory_order_relaxed);
-  long long want = std::max<long long>(3, ((n + 3) / 4 + lanes_per_sm - 1) / lanes_per_sm);
-  if (fixed > 0) want = fixed;
-  else if (std::is_same<T, float>::value) want = per_sm;
+  const long long want = fixed > 0 ? fixed : sq_fwd_want(n, sms);
   const long long need = (n + SQF_T - 1) / SQF_T;
   const int fblocks = (int)std::max<long long>(
       1, std::min<long long>((long long)sms * std::min<long long>(std::max(per_sm, 1), want), need));
@@ -2890,13 +2890,15 @@ cudaError_t launch_sq_energy_batch(const SqBatchReq* r, int K, void* scratch, do
   o.seed_L = reinterpret_cast<float*>(scr + L.seed_L);
   o.ck = reinterpret_cast<V4<float>*>(scr + L.ck);
   o.applied = work;
-  // persistent forward grid: the resident blocks, as the single call
+  // persistent forward grid, as the single call's
   int per_sm = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sq_fwd_batch_kernel, SQF_T, 0)))
     return e;
   const long long need = (L.n_flat + SQF_T - 1) / SQF_T;
   const int fblocks = (int)std::max<long long>(
-      1, std::min<long long>((long long)sms * std::max(per_sm, 1), need));
+      1, std::min<long long>((long long)sms * std::min<long long>(std::max(per_sm, 1),
+                                                                 sq_fwd_want(L.n_flat, sms)),
+                            need));
   sq_fwd_batch_kernel<<<fblocks, SQF_T, 0, s>>>(d_items, d_chunk_item, L.n_flat, claim, o);
   n_launch++;
   // per item: chunk sums and histogram, the sort's scan and scatter
