@@ -171,17 +171,21 @@ __device__ __forceinline__ Q qpow_cr(const Q& q, double e) {
   return o;
 }
 
-// Integer power by repeated products (exact algebra, FP64 rounding).
+// Integer power by repeated products (exact algebra, FP64 rounding).  In the
+// reference's order like every product of the FP64 chain: with fused products
+// a pair of conjugate factors left a vector part of 2^-54 where these cancel
+// it exactly, and the orbits left the real axis (33 of 6500 points on it had
+// the other sign after 40 applications, 100 maps of one pair and one real
+// root).
 __device__ __forceinline__ Q qpow_int(const Q& d, int n) {
   Q r = d;
   for (int k = 1; k < n; k++) r = qmul(r, d);
   return r;
 }
 
-// The products of the integer-power form, which follows no reference
-// rounding: fused multiply-adds, 16 instructions of the FP64 pipe (1/64 of
-// the FP32 rate, its throughput is what bounds every FP64 kernel here) in
-// place of qmul's 28, and one rounding less in each of 12 places.
+// Fused products, where no reference rounding is followed and no term has to
+// cancel exactly (the optimizer's gradient): 16 instructions of the FP64 pipe
+// in place of qmul's 28.
 __device__ __forceinline__ Q fmul(const Q& a, const Q& b) {
   Q o;
   o.w = fma(-a.z, b.z, fma(-a.y, b.y, fma(-a.x, b.x, mul(a.w, b.w))));
@@ -189,12 +193,6 @@ __device__ __forceinline__ Q fmul(const Q& a, const Q& b) {
   o.y = fma(a.z, b.x, fma(a.y, b.w, fma(-a.x, b.z, mul(a.w, b.y))));
   o.z = fma(a.z, b.w, fma(-a.y, b.x, fma(a.x, b.y, mul(a.w, b.z))));
   return o;
-}
-
-__device__ __forceinline__ Q fsq(const Q& a) {
-  const double w2 = add(a.w, a.w);
-  return Q{fma(-a.z, a.z, fma(-a.y, a.y, fma(-a.x, a.x, mul(a.w, a.w)))), mul(w2, a.x),
-           mul(w2, a.y), mul(w2, a.z)};
 }
 
 __device__ __forceinline__ double fnorm2(const Q& q) {
@@ -205,13 +203,6 @@ __device__ __forceinline__ double fnorm2(const Q& q) {
 __device__ __forceinline__ Q fdiv(const Q& l, const Q& r) {
   const double inv = __ddiv_rn(1.0, fnorm2(r));
   return fmul(l, Q{mul(r.w, inv), mul(-r.x, inv), mul(-r.y, inv), mul(-r.z, inv)});
-}
-
-__device__ __forceinline__ Q fpow(const Q& d, int n) {
-  if (n == 1) return d;
-  Q r = fsq(d);
-  for (int k = 2; k < n; k++) r = fmul(r, d);
-  return r;
 }
 
 __device__ __forceinline__ bool same_bits(double a, double b) {
@@ -467,19 +458,7 @@ __device__ __forceinline__ q64::Q term64(const MapParams& m, const q64::Q& q, in
     g.y += k * d.y;
     g.z += k * d.z;
   }
-  return POW_REF == 2 ? qpow_cr(d, m.e64[i]) : POW_REF ? qpow(d, m.e64[i]) : fpow(d, m.ie[i]);
-}
-
-// The FP64 chain's product and quotient (the Lagrange order, the correctly
-// rounded functions, maps out of quotient_fx's range): reference order and
-// rounding for the polar powers, fused for the integer ones.
-template <int POW_REF>
-__device__ __forceinline__ q64::Q times64(const q64::Q& a, const q64::Q& b) {
-  return POW_REF ? q64::qmul(a, b) : q64::fmul(a, b);
-}
-template <int POW_REF>
-__device__ __forceinline__ q64::Q over64(const q64::Q& a, const q64::Q& b) {
-  return POW_REF ? q64::qdiv(a, b) : q64::fdiv(a, b);
+  return POW_REF == 2 ? qpow_cr(d, m.e64[i]) : POW_REF ? qpow(d, m.e64[i]) : qpow_int(d, m.ie[i]);
 }
 
 template <int POW_REF, bool DE>
@@ -490,7 +469,7 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
 #pragma unroll 1
   for (int i = lo; i < hi; i++) {
     const Q t = term64<POW_REF, DE>(m, q, i, sign, g);
-    r = (i == lo) ? t : times64<POW_REF>(r, t);
+    r = (i == lo) ? t : qmul(r, t);
   }
   return r;
 }
@@ -563,7 +542,7 @@ __device__ __forceinline__ q64::Q quotient64(const MapParams& m, const q64::Q& q
   g = q64::Q{0.0, 0.0, 0.0, 0.0};
   const q64::Q top = product64<POW_REF, DE>(m, q, 0, m.nt, 1.0, g);
   if (m.nb == 0) return top;
-  return over64<POW_REF>(top, product64<POW_REF, DE>(m, q, m.nt, m.nt + m.nb, -1.0, g));
+  return q64::qdiv(top, product64<POW_REF, DE>(m, q, m.nt, m.nt + m.nb, -1.0, g));
 }
 template <int POW_REF, bool DE>
 static __device__ __noinline__ q64::Q quotient64_far(const MapParams& m, const q64::Q q,
@@ -582,13 +561,13 @@ __device__ __forceinline__ q64::Q lagrange64(const MapParams& m, const q64::Q& q
   const int same = m.nt < m.nb ? m.nt : m.nb;
 #pragma unroll 1
   for (int k = 0; k < same; k++) {
-    r = times64<POW_REF>(r, term64<POW_REF, DE>(m, q, k, 1.0, g));
-    r = over64<POW_REF>(r, term64<POW_REF, DE>(m, q, m.nt + k, -1.0, g));
+    r = qmul(r, term64<POW_REF, DE>(m, q, k, 1.0, g));
+    r = qdiv(r, term64<POW_REF, DE>(m, q, m.nt + k, -1.0, g));
   }
 #pragma unroll 1
-  for (int k = same; k < m.nt; k++) r = times64<POW_REF>(r, term64<POW_REF, DE>(m, q, k, 1.0, g));
+  for (int k = same; k < m.nt; k++) r = qmul(r, term64<POW_REF, DE>(m, q, k, 1.0, g));
 #pragma unroll 1
-  for (int k = same; k < m.nb; k++) r = over64<POW_REF>(r, term64<POW_REF, DE>(m, q, m.nt + k, -1.0, g));
+  for (int k = same; k < m.nb; k++) r = qdiv(r, term64<POW_REF, DE>(m, q, m.nt + k, -1.0, g));
   return r;
 }
 
