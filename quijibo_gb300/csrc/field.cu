@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128) field64_kernel(const __grid_constant__ Ma
 // distance estimate (26 of 50 FP64 instructions of a root term with exponent
 // 1) only where the caller wants it.
 template <int POW_REF, bool DE>
-__global__ void __launch_bounds__(128) refine64_kernel(const __grid_constant__ MapParams m,
+__global__ void __launch_bounds__(128, DE ? 3 : 4) refine64_kernel(const __grid_constant__ MapParams m,
                                                        const GridParams g,
                                                        const IterParams it, const uint32_t* list,
                                                        const DevStats* counts,

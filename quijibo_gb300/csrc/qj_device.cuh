@@ -199,12 +199,6 @@ __device__ __forceinline__ double fnorm2(const Q& q) {
   return fma(q.z, q.z, fma(q.y, q.y, fma(q.x, q.x, mul(q.w, q.w))));
 }
 
-// l * conj(r) / |r|^2
-__device__ __forceinline__ Q fdiv(const Q& l, const Q& r) {
-  const double inv = __ddiv_rn(1.0, fnorm2(r));
-  return fmul(l, Q{mul(r.w, inv), mul(-r.x, inv), mul(-r.y, inv), mul(-r.z, inv)});
-}
-
 __device__ __forceinline__ bool same_bits(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b);
 }
@@ -475,24 +469,33 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
 }
 
 // The quotient of the sides' products, the products in fixed point
-// (qj_fxmath.h); *odd where a term or a partial product leaves [2^-500,
-// 2^500], zero or not finite: there the FP64 chain's own overflow, underflow
-// and NaN count.  The FP64 pipe issues 1/64 of what the integer
-// pipe does: as fused FP64 products the refine pass over a 128^3 grid whose
-// inside needs it held that pipe at 80% for 46 ms, as these it takes 11.7 ms
-// (FP64 20%, ALU 62% busy); calls that mesh 128^3 grids, one of three like
-// that, went 24.5 -> 11.1 ms on average.  The polar powers' products, 28 of
-// a term's 52 FP64 instructions in the reference's order: plain FP64 field
-// 64^3 6.7 -> 4.6 ms, FP64 mesh 48^3 9.2 -> 6.1 ms (12 / 6 roots; 5.3 and
-// 6.9 ms with a loop for each side and the FP64 chain expanded in place: the
-// code has to stay small for instruction fetch).  The product of 24 factors
-// is off by 0.45 units of 2^-53 (rms), the fused one by 3.8.
+// (qj_fxmath.h); *odd where the FP64 chain's own products are wanted: a term
+// or a partial product leaves [2^-500, 2^500], zero or not finite (its
+// overflow, underflow and NaN), or a component is small in all its terms or
+// the vector part as a whole, on and beside the real axis and coordinate
+// planes (fx_quat's odd; 2e-5 to 4e-4 of the applications over maps with
+// generic roots).  Without that test the orbits of q^3 + c left the real axis:
+// 23 of 33 points on it had the other sign.
+// The FP64 pipe issues 1/64 of what the integer pipe does: as fused FP64
+// products the refine pass over a 128^3 grid whose inside needs it held that
+// pipe at 80% for 46 ms, as these it takes 11.7 ms; calls that mesh 128^3
+// grids, one of three like that, went 24.5 -> 11.1 ms on average.  The polar
+// powers' products, 28 of a term's 52 FP64 instructions in the reference's
+// order: plain FP64 field 64^3 6.7 -> 4.5 ms, FP64 mesh 48^3 9.2 -> 6.1 ms
+// (12 / 6 roots; 5.3 and 6.9 ms with a loop for each side and the FP64 chain
+// expanded in place: the code has to stay small for instruction fetch).  The
+// tests and the cut of magnitudes cost what the roots' common exponent and
+// the division in fixed point give back where the pipes are full (one refine
+// pass 5.17 -> 5.03 ms, FP64 15%, ALU 56% busy), and 5-10% where one warp's
+// chain is waited for (32^3 field 353 -> 372 us).  The product of 24 factors
+// is off by 0.55 units of 2^-53 (rms), the fused one by 3.8.
 template <int POW_REF, bool DE>
 __device__ __forceinline__ q64::Q quotient_fx(const MapParams& m, const q64::Q& q, q64::Q& g,
                                               bool* odd) {
   using namespace q64;
   fx_quat qx, r, top;
-  if (POW_REF == 0) qx = fx_quat_of(q.w, q.x, q.y, q.z);
+  if (POW_REF == 0)
+    qx = fx_quat_at(q.w, q.x, q.y, q.z, max(m.afx, fx_top(q.w, q.x, q.y, q.z)));
   const int nt = m.nt, n = nt + m.nb;
 #pragma unroll 1
   for (int i = 0; i < n; i++) {
@@ -513,27 +516,46 @@ __device__ __forceinline__ q64::Q quotient_fx(const MapParams& m, const q64::Q& 
       const Q p = qpow(d, m.e64[i]);
       t = fx_quat_of(p.w, p.x, p.y, p.z);
     } else {
-      const fx_quat root{m.rfx[i][0], m.rfx[i][1], m.rfx[i][2], m.rfx[i][3], m.efx[i]};
+      fx_quat root;
+      root.w = m.rfx[i][0];
+      root.x = m.rfx[i][1];
+      root.y = m.rfx[i][2];
+      root.z = m.rfx[i][3];
+      root.e = m.efx[i];
       fx_quat b = fx_qsub(qx, root);
-      if (fx_near(b, qx, root))  // rare: FP64's own difference keeps the low bits
+      // rare: FP64's own difference keeps the low bits, those of a small
+      // component too, unless it is exactly zero
+      bool near = fx_near(b, qx, root);
+      if (b.odd)
+        near = near || (b.odd & 1 && q.w != m.r64[i][0]) || (b.odd & 2 && q.x != m.r64[i][1]) ||
+               (b.odd & 4 && q.y != m.r64[i][2]) || (b.odd & 8 && q.z != m.r64[i][3]);
+      b.odd = 0;
+      if (near)
         b = fx_quat_of(sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
                        sub(q.z, m.r64[i][3]));
       const int e = m.ie[i];
       t = b;
       if (e > 1) t = fx_qsq(b);
-      for (int k = 2; k < e; k++) t = fx_qmul(t, b);
+      for (int k = 2; k < e; k++) t = fx_qpower(t, b);
     }
     if (i == nt) top = r;
     r = i == 0 || i == nt ? t : fx_qmul(r, t);
-    *odd |= (unsigned)(t.e + 500) > 1000u || (unsigned)(r.e + 500) > 1000u;
+    *odd |= (unsigned)(t.e + 500) > 1000u || (unsigned)(r.e + 500) > 1000u || t.odd || r.odd;
   }
-  Q out{(double)r.w, (double)r.x, (double)r.y, (double)r.z};
   int k = r.e - 62;
+  double inv = 1.0;
   if (n > nt) {
-    out = fdiv(Q{(double)top.w, (double)top.x, (double)top.y, (double)top.z}, out);
-    k = top.e - r.e;
+    // top conj(r) / |r|^2
+    inv = __ddiv_rn(1.0, fnorm2(Q{(double)r.mw, (double)r.mx, (double)r.my, (double)r.mz}));
+    k = 62 - 2 * r.e;
+    r = fx_qmul(top, fx_conj(r));
+    k += r.e;
+    *odd |= r.odd;
   }
-  return Q{fx_scale(out.w, k), fx_scale(out.x, k), fx_scale(out.y, k), fx_scale(out.z, k)};
+  *odd |= n == 1;  // (no product's test)
+  r = fx_joined(r);
+  return Q{fx_scale(mul((double)r.w, inv), k), fx_scale(mul((double)r.x, inv), k),
+           fx_scale(mul((double)r.y, inv), k), fx_scale(mul((double)r.z, inv), k)};
 }
 
 // The same by the FP64 chain.

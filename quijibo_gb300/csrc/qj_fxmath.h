@@ -363,79 +363,221 @@ FX_FN void fx_sincos(double x, double* sn, double* cs) {
 }
 
 // ---- quaternion products in fixed point ---------------------------------
-// A Hamilton product costs 16 FP64 instructions, as much of that pipe's time
-// as 1024 integer ones would take on theirs.  Here a quaternion is four
-// 64-bit integers with one exponent, value c 2^(e - 62), the largest |c| in
-// [2^61, 2^62): a product is 16 high halves of 64-bit products and a
-// renormalization, about 230 integer instructions.  Against |a b| it is off
-// by at most 2^-55 (four truncated halves, and the largest component of a
-// product of norm 2^58 is at least 2^57), FP64's fused product by 2^-52.
+// A Hamilton product costs 28 FP64 instructions in the reference's order, as
+// much of that pipe's time as 1792 integer ones would take on theirs.  Here a
+// quaternion is four 64-bit integers with one exponent, value c 2^(e - 62),
+// the largest |c| in [2^61, 2^62): a product is 16 high halves of 64-bit
+// products of magnitudes and a renormalization.  Against |a b| it is off by
+// at most 2^-55 (four halves cut towards 0, and the largest component of a
+// product of norm 2^58 is at least 2^57), an FP64 product by 2^-52.
+//
+// Every step cuts magnitudes, so that values of opposite sign are treated
+// alike: terms that cancel exactly in FP64 (conjugate factors) cancel here,
+// and mirror images have the same bits.  The error is one of the whole
+// quaternion, FP64's of each component.  Where a component is small in every
+// one of its terms (near the real axis or a coordinate plane with roots in
+// it), FP64 keeps it to 2^-53 of itself, and whether it is zero decides the
+// polar power's branch: `odd` then says that FP64's product is wanted, as
+// soon as all four terms of a component are below 2^-9 of the largest they
+// could be without all being zero, or the vector part as a whole is.
 typedef struct {
-  fx_i64 w, x, y, z;
+  fx_i64 w, x, y, z;       // the components, and as magnitude and sign (0 or
+  fx_u64 mw, mx, my, mz;   // -1): the compiler drops what a caller leaves
+  int32_t sw, sx, sy, sz;  // unused
   int e;
+  int odd;  // not held as FP64 would hold it (of a difference: bit c, component c is small)
 } fx_quat;
 
+FX_FN uint32_t fx_high(fx_u64 v) { return (uint32_t)(v >> 32); }
+FX_FN uint32_t fx_least(uint32_t a, uint32_t b) { return a < b ? a : b; }
+// the sign of c, and a sign in both halves of a word
+FX_FN int32_t fx_sign(fx_i64 c) { return (int32_t)(c >> 32) >> 31; }
+FX_FN fx_u64 fx_mask(int32_t s) {
+#ifdef __CUDACC__
+  fx_u64 m;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(m) : "r"(s));
+  return m;
+#else
+  return (fx_u64)(fx_i64)s;
+#endif
+}
+FX_FN fx_u64 fx_abs(fx_i64 c) {
+  const fx_u64 s = fx_mask(fx_sign(c));
+  return ((fx_u64)c ^ s) - s;
+}
+FX_FN fx_i64 fx_signed(fx_u64 m, int32_t s) { return (fx_i64)((m ^ fx_mask(s)) - fx_mask(s)); }
+// v 2^-s, its magnitude cut; 0 <= s < 64
+FX_FN fx_i64 fx_cut(fx_i64 v, int s) { return fx_signed(fx_abs(v) >> s, fx_sign(v)); }
+
+// magnitudes and signs from the components, and back
+FX_FN fx_quat fx_split(fx_quat q) {
+  q.sw = fx_sign(q.w);
+  q.sx = fx_sign(q.x);
+  q.sy = fx_sign(q.y);
+  q.sz = fx_sign(q.z);
+  q.mw = fx_abs(q.w);
+  q.mx = fx_abs(q.x);
+  q.my = fx_abs(q.y);
+  q.mz = fx_abs(q.z);
+  return q;
+}
+FX_FN fx_quat fx_joined(fx_quat q) {
+  q.w = fx_signed(q.mw, q.sw);
+  q.x = fx_signed(q.mx, q.sx);
+  q.y = fx_signed(q.my, q.sy);
+  q.z = fx_signed(q.mz, q.sz);
+  return q;
+}
+// The largest magnitude's top bit to 2^61; none is 2^62 or more.
+FX_FN fx_quat fx_norm(fx_quat q) {
+  const fx_u64 any = q.mw | q.mx | q.my | q.mz;
+  const int s = any ? fx_clz(any) - 2 : 61;
+  q.mw <<= s;
+  q.mx <<= s;
+  q.my <<= s;
+  q.mz <<= s;
+  q.e -= s;
+  return fx_joined(q);
+}
+
+FX_FN int fx_field(double v) { return (int)(fx_bits(v) >> 52) & 0x7ff; }
 // v's mantissa in units of 2^(top - 62), top at least v's exponent; 0 for
 // zeros and subnormals.
-FX_FN fx_i64 fx_align(double v, int top) {
-  const fx_u64 b = fx_bits(v);
-  const int f = (int)(b >> 52) & 0x7ff;
-  const int sh = 2 + top - (f - 1022);
-  if (f == 0 || sh > 63) return 0;
-  const fx_i64 m = (fx_i64)(((b << 11) | 0x8000000000000000ull) >> sh);
-  return (fx_i64)b < 0 ? -m : m;
+FX_FN fx_u64 fx_align(double v, int top) {
+  const int f = fx_field(v), sh = 2 + top - (f - 1022);
+  return f == 0 || sh > 63 ? 0 : ((fx_bits(v) << 11) | 0x8000000000000000ull) >> sh;
 }
-FX_FN fx_quat fx_quat_of(double w, double x, double y, double z) {
-  int f = (int)(fx_bits(w) >> 52) & 0x7ff, g = (int)(fx_bits(x) >> 52) & 0x7ff;
+// The exponent of the largest component.
+FX_FN int fx_top(double w, double x, double y, double z) {
+  int f = fx_field(w), g = fx_field(x);
   f = f > g ? f : g;
-  g = (int)(fx_bits(y) >> 52) & 0x7ff;
+  g = fx_field(y);
   f = f > g ? f : g;
-  g = (int)(fx_bits(z) >> 52) & 0x7ff;
-  f = f > g ? f : g;
+  g = fx_field(z);
+  return (f > g ? f : g) - 1022;
+}
+// The components in units of 2^(top - 62), top at least fx_top's.
+FX_FN fx_quat fx_quat_at(double w, double x, double y, double z, int top) {
   fx_quat q;
-  q.e = f - 1022;
-  q.w = fx_align(w, q.e);
-  q.x = fx_align(x, q.e);
-  q.y = fx_align(y, q.e);
-  q.z = fx_align(z, q.e);
+  q.e = top;
+  q.odd = 0;
+  q.sw = fx_sign((fx_i64)fx_bits(w));
+  q.sx = fx_sign((fx_i64)fx_bits(x));
+  q.sy = fx_sign((fx_i64)fx_bits(y));
+  q.sz = fx_sign((fx_i64)fx_bits(z));
+  q.mw = fx_align(w, top);
+  q.mx = fx_align(x, top);
+  q.my = fx_align(y, top);
+  q.mz = fx_align(z, top);
+  return fx_joined(q);
+}
+// odd where a component that is not zero has fewer than 11 bits left
+FX_FN fx_quat fx_quat_of(double w, double x, double y, double z) {
+  const int top = fx_top(w, x, y, z), least = top + 1022 - 51;
+  fx_quat q = fx_quat_at(w, x, y, z, top);
+  if (fx_field(w) < least || fx_field(x) < least || fx_field(y) < least || fx_field(z) < least)
+    q.odd = (w != 0.0 && fx_field(w) < least) || (x != 0.0 && fx_field(x) < least) ||
+            (y != 0.0 && fx_field(y) < least) || (z != 0.0 && fx_field(z) < least);
   return q;
 }
-FX_FN fx_quat fx_norm(fx_quat q) {
-  // the bits of |c| - 1 or |c|: enough to place the top bit (none: 0 or -1)
-  const fx_u64 any = (fx_u64)((q.w ^ q.w >> 63) | (q.x ^ q.x >> 63) | (q.y ^ q.y >> 63) |
-                              (q.z ^ q.z >> 63));
-  const int s = any ? fx_clz(any) - 2 : 61;
-  q.w = (fx_i64)((fx_u64)q.w << s);
-  q.x = (fx_i64)((fx_u64)q.x << s);
-  q.y = (fx_i64)((fx_u64)q.y << s);
-  q.z = (fx_i64)((fx_u64)q.z << s);
-  q.e -= s;
-  return q;
-}
-// a - b, each kept to 2^-61 of the larger one's largest component: off by
-// at most 2^-53 of |a - b| unless fx_near says that more bits cancelled.
+
+// a - b, each kept to 2^-62 of the larger exponent: off by at most 2^-53 of
+// |a - b| unless fx_near says that more bits cancelled.  odd: bit c where
+// component c has fewer than 33 bits; such a one is exact where the operands'
+// components are equal.  (Of the operands only w to z and e count.)
 FX_FN fx_quat fx_qsub(fx_quat a, fx_quat b) {
   fx_quat o;
-  o.e = (a.e > b.e ? a.e : b.e) + 1;
-  const int sa = o.e - a.e < 63 ? o.e - a.e : 63, sb = o.e - b.e < 63 ? o.e - b.e : 63;
-  o.w = (a.w >> sa) - (b.w >> sb);
-  o.x = (a.x >> sa) - (b.x >> sb);
-  o.y = (a.y >> sa) - (b.y >> sb);
-  o.z = (a.z >> sa) - (b.z >> sb);
-  return fx_norm(o);
+  o.e = a.e > b.e ? a.e : b.e;
+  if (a.e != b.e) {
+    const int sa = o.e - a.e < 63 ? o.e - a.e : 63, sb = o.e - b.e < 63 ? o.e - b.e : 63;
+    a.w = fx_cut(a.w, sa);
+    a.x = fx_cut(a.x, sa);
+    a.y = fx_cut(a.y, sa);
+    a.z = fx_cut(a.z, sa);
+    b.w = fx_cut(b.w, sb);
+    b.x = fx_cut(b.x, sb);
+    b.y = fx_cut(b.y, sb);
+    b.z = fx_cut(b.z, sb);
+  }
+  o.w = a.w - b.w;
+  o.x = a.x - b.x;
+  o.y = a.y - b.y;
+  o.z = a.z - b.z;
+  o = fx_split(o);
+  o.odd = (fx_high(o.mw) == 0) | (fx_high(o.mx) == 0) << 1 | (fx_high(o.my) == 0) << 2 |
+          (fx_high(o.mz) == 0) << 3;
+  // below 2^63: the top bit to 2^62, then half
+  const fx_u64 any = o.mw | o.mx | o.my | o.mz;
+  const int s = any ? fx_clz(any) - 1 : 62;
+  o.mw = o.mw << s >> 1;
+  o.mx = o.mx << s >> 1;
+  o.my = o.my << s >> 1;
+  o.mz = o.mz << s >> 1;
+  o.e -= s - 1;
+  return fx_joined(o);
 }
 // Whether d = fx_qsub(a, b) came out below 2^-6 of the larger of a and b.
 FX_FN int fx_near(fx_quat d, fx_quat a, fx_quat b) {
   return d.e < (a.e > b.e ? a.e : b.e) - 5;
 }
-FX_FN fx_quat fx_qmul(fx_quat a, fx_quat b) {
+
+// m with sign s but for the 1 that a negative one lacks
+FX_FN fx_u64 fx_flip(fx_u64 m, int32_t s) { return m ^ fx_mask(s); }
+// The sum of four products of magnitudes, each cut, with signs s1 to s4.
+FX_FN fx_i64 fx_sum4(fx_u64 a1, fx_u64 b1, int32_t s1, fx_u64 a2, fx_u64 b2, int32_t s2, fx_u64 a3,
+                     fx_u64 b3, int32_t s3, fx_u64 a4, fx_u64 b4, int32_t s4) {
+  const uint32_t minus = (uint32_t)-(s1 + s2 + s3 + s4);
+  return (fx_i64)(fx_flip(fx_mulhi(a1, b1), s1) + fx_flip(fx_mulhi(a2, b2), s2) +
+                  fx_flip(fx_mulhi(a3, b3), s3) + fx_flip(fx_mulhi(a4, b4), s4) + minus);
+}
+// Whether all four terms are below 2^51 of at most 2^60 (by the high halves)
+// and not all zero.
+FX_FN int fx_lost(fx_u64 a1, fx_u64 b1, fx_u64 a2, fx_u64 b2, fx_u64 a3, fx_u64 b3, fx_u64 a4,
+                  fx_u64 b4) {
+  const fx_u64 most = (fx_u64)fx_high(a1) * fx_high(b1) | (fx_u64)fx_high(a2) * fx_high(b2) |
+                      (fx_u64)fx_high(a3) * fx_high(b3) | (fx_u64)fx_high(a4) * fx_high(b4);
+  return most < (1ull << 51) && ((a1 && b1) || (a2 && b2) || (a3 && b3) || (a4 && b4));
+}
+// The product; `strict`: of two factors of the map, odd as said above.
+FX_FN fx_quat fx_hamilton(fx_quat a, fx_quat b, int strict) {
   fx_quat o;
-  o.w = fx_smulhi(a.w, b.w) - fx_smulhi(a.x, b.x) - fx_smulhi(a.y, b.y) - fx_smulhi(a.z, b.z);
-  o.x = fx_smulhi(a.w, b.x) + fx_smulhi(a.x, b.w) + fx_smulhi(a.y, b.z) - fx_smulhi(a.z, b.y);
-  o.y = fx_smulhi(a.w, b.y) - fx_smulhi(a.x, b.z) + fx_smulhi(a.y, b.w) + fx_smulhi(a.z, b.x);
-  o.z = fx_smulhi(a.w, b.z) + fx_smulhi(a.x, b.y) - fx_smulhi(a.y, b.x) + fx_smulhi(a.z, b.w);
+  o.w = fx_sum4(a.mw, b.mw, a.sw ^ b.sw, a.mx, b.mx, ~(a.sx ^ b.sx), a.my, b.my, ~(a.sy ^ b.sy),
+                a.mz, b.mz, ~(a.sz ^ b.sz));
+  o.x = fx_sum4(a.mw, b.mx, a.sw ^ b.sx, a.mx, b.mw, a.sx ^ b.sw, a.my, b.mz, a.sy ^ b.sz, a.mz,
+                b.my, ~(a.sz ^ b.sy));
+  o.y = fx_sum4(a.mw, b.my, a.sw ^ b.sy, a.mx, b.mz, ~(a.sx ^ b.sz), a.my, b.mw, a.sy ^ b.sw, a.mz,
+                b.mx, a.sz ^ b.sx);
+  o.z = fx_sum4(a.mw, b.mz, a.sw ^ b.sz, a.mx, b.my, a.sx ^ b.sy, a.my, b.mx, ~(a.sy ^ b.sx), a.mz,
+                b.mw, a.sz ^ b.sw);
   o.e = a.e + b.e + 2;
-  return fx_norm(o);
+  o.odd = a.odd | b.odd;
+  o = fx_norm(fx_split(o));
+  if (strict) {
+    // no small component on one side: its product with the other side's
+    // largest is a term of 2^51 or more in every component
+    const uint32_t p = fx_least(fx_least(fx_high(a.mw), fx_high(a.mx)), fx_least(fx_high(a.my), fx_high(a.mz)));
+    const uint32_t q = fx_least(fx_least(fx_high(b.mw), fx_high(b.mx)), fx_least(fx_high(b.my), fx_high(b.mz)));
+    const int real = fx_high(o.mx | o.my | o.mz) < (1u << 21);
+    if ((p < (1u << 22) && q < (1u << 22)) || real)
+      o.odd |= (real && ((a.mx | a.my | a.mz) || (b.mx | b.my | b.mz))) ||
+               fx_lost(a.mw, b.mw, a.mx, b.mx, a.my, b.my, a.mz, b.mz) ||
+               fx_lost(a.mw, b.mx, a.mx, b.mw, a.my, b.mz, a.mz, b.my) ||
+               fx_lost(a.mw, b.my, a.mx, b.mz, a.my, b.mw, a.mz, b.mx) ||
+               fx_lost(a.mw, b.mz, a.mx, b.my, a.my, b.mx, a.mz, b.mw);
+  }
+  return o;
+}
+// The product of two factors of the map.
+FX_FN fx_quat fx_qmul(fx_quat a, fx_quat b) { return fx_hamilton(a, b, 1); }
+// ... and of a power and its base.  Their vectors are parallel, so the terms
+// of a component are small together on a 2^-8 of all bases; a later factor's
+// terms then count beside them, and the product with it is tested.
+FX_FN fx_quat fx_qpower(fx_quat a, fx_quat b) { return fx_hamilton(a, b, 0); }
+FX_FN fx_quat fx_conj(fx_quat a) {
+  a.sx = ~a.sx;
+  a.sy = ~a.sy;
+  a.sz = ~a.sz;
+  return fx_joined(a);
 }
 // v 2^k for a normal result, by the exponent field (0, infinities and NaN stay).
 FX_FN double fx_scale(double v, int k) {
@@ -446,12 +588,22 @@ FX_FN double fx_scale(double v, int k) {
   if (f + k >= 0x7ff) return fx_from((b & 0x8000000000000000ull) | 0x7ff0000000000000ull);
   return fx_from(b + ((fx_u64)(fx_i64)k << 52));
 }
+// odd where a component 2 w c has fewer than 33 bits and is not zero
 FX_FN fx_quat fx_qsq(fx_quat a) {
   fx_quat o;
-  o.w = fx_smulhi(a.w, a.w) - fx_smulhi(a.x, a.x) - fx_smulhi(a.y, a.y) - fx_smulhi(a.z, a.z);
-  o.x = fx_smulhi(a.w << 1, a.x);
-  o.y = fx_smulhi(a.w << 1, a.y);
-  o.z = fx_smulhi(a.w << 1, a.z);
+  o.w = (fx_i64)(fx_mulhi(a.mw, a.mw) - fx_mulhi(a.mx, a.mx) - fx_mulhi(a.my, a.my) -
+                 fx_mulhi(a.mz, a.mz));
+  o.sw = fx_sign(o.w);
+  o.mw = fx_abs(o.w);
+  o.mx = fx_mulhi(a.mw << 1, a.mx);
+  o.my = fx_mulhi(a.mw << 1, a.my);
+  o.mz = fx_mulhi(a.mw << 1, a.mz);
+  o.sx = a.sw ^ a.sx;
+  o.sy = a.sw ^ a.sy;
+  o.sz = a.sw ^ a.sz;
+  o.odd = a.odd;
+  if (fx_least(fx_high(o.mx), fx_least(fx_high(o.my), fx_high(o.mz))) == 0)
+    o.odd |= a.mw && ((a.mx && !fx_high(o.mx)) || (a.my && !fx_high(o.my)) || (a.mz && !fx_high(o.mz)));
   o.e = a.e + a.e + 2;
   return fx_norm(o);
 }

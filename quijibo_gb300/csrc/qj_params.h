@@ -34,9 +34,10 @@ struct MapParams {
   alignas(16) float2 rn2[QJ_MAX_ROOTS][4];  // (-t_c, -t_c) for c = w, x, y, z
   alignas(8) float2 ex2[QJ_MAX_ROOTS];      // (x32[i][0], x32[i][0])
   // the FP64 form's integer powers: each root as a fixed-point quaternion
-  // (fx_quat of qj_fxmath.h)
+  // (fx_quat_at of qj_fxmath.h) and the exponent that most of them share
   alignas(16) long long rfx[QJ_MAX_ROOTS][4];
   int efx[QJ_MAX_ROOTS];
+  int afx;
   // the double-float head: each root coordinate and the scale as hi + lo
   alignas(8) float rff[QJ_MAX_ROOTS][4][2];
   float scale_ff[2];

@@ -100,3 +100,43 @@ def test_integer_powers_in_the_lagrange_order(ctx, seed, nb, max_it):
     rs = conjugate_map(seed, nb)
     _assert_same(_integer_form(ctx, rs, LINE, max_it, True),
                  _field(rs, _start(LINE), max_it, 2.0, True))
+
+
+@pytest.mark.parametrize("max_it", [1, 40])
+@pytest.mark.parametrize("seed,nb", [(0, 0), (100, 0), (112, 0), (1, 1), (3, 3), (32, 3), (65, 3)])
+def test_integer_powers(ctx, seed, nb, max_it):
+    rs = conjugate_map(seed, nb)
+    f, want = _integer_form(ctx, rs, LINE, max_it, False), _field(rs, _start(LINE), max_it, 2.0, False)
+    if nb == 1:  # half a pair below: off the axis from the first step, no exact cancellation
+        assert (np.abs(f - want) <= 1e-9 * (1 + np.abs(want))).all()
+    else:
+        _assert_same(f, want)
+
+
+def _assert_polar_forms(ctx, oracle, rs, g):
+    """One last-bit change in every power leaves these fields within 1e-6;
+    a vector part of 2^-61 changes the sign of up to two thirds of them."""
+    o = oracle.field(rs, g, 40, 2.0)["field"]
+    h = ctx.upload(rs)
+    for it in (ctx.iter_params(40, 2.0),
+               ctx.iter_params(40, 2.0, precision=lib.QJG_FP32_REFINE, rel_tol=1e-30)):
+        f = ctx.field_host(h, g, it)[0]
+        assert np.array_equal(f > 0, o > 0)
+        assert (np.abs(f - o) <= 1e-6 * (1 + np.abs(o))).all()
+    ctx.free(h)
+
+
+@pytest.mark.parametrize("seed,nb", [(11, 0), (13, 0), (18, 0), (19, 0), (1, 3), (14, 3), (16, 3), (18, 3), (32, 3)])
+def test_polar_powers(ctx, oracle, seed, nb):
+    _assert_polar_forms(ctx, oracle, conjugate_map(seed, nb), LINE)
+
+
+@pytest.mark.parametrize("g", [Grid((33, 1, 1)), Grid((21, 21, 21))])
+@pytest.mark.parametrize("c", [-0.6, -1.2])
+def test_cubic(ctx, oracle, c, g):
+    """q^3 + c, the pair before the real root; on the odd cube the axis cells
+    have y and z a rounding off 0."""
+    z = np.roots([1, 0, 0, c])
+    pair, real = z[z.imag > 1e-9][0], z[abs(z.imag) < 1e-9][0].real
+    top = [[pair.real, pair.imag, 0, 0], [pair.real, -pair.imag, 0, 0], [real, 0, 0, 0]]
+    _assert_polar_forms(ctx, oracle, RootSet(top_roots=np.array(top), top_powers=np.ones(3)), g)
