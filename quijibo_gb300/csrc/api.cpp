@@ -152,7 +152,7 @@ int qj_fill_map(MapParams* m, int n_top, const double* top_roots, const double* 
   m->sigma[0] = sigma_top;
   m->sigma[1] = sigma_bot;
   m->all_int = 1;
-  std::vector<int> top_exp;
+  int top_exp[QJ_MAX_ROOTS], sorted[QJ_MAX_ROOTS];
   for (int i = 0; i < n_top + n_bot; i++) {
     const bool top = i < n_top;
     const double* r = top ? top_roots + 4 * i : bot_roots + 4 * (i - n_top);
@@ -168,7 +168,7 @@ int qj_fill_map(MapParams* m, int n_top, const double* top_roots, const double* 
       m->rff[i][c][0] = m->r32[i][c];
       m->rff[i][c][1] = (float)(r[c] - (double)m->r32[i][c]);
     }
-    top_exp.push_back(fx_top(r[0], r[1], r[2], r[3]));
+    top_exp[i] = sorted[i] = fx_top(r[0], r[1], r[2], r[3]);
     m->e64[i] = e;
     m->ep[i] = pw;
     m->e32[i] = (float)e;
@@ -183,13 +183,12 @@ int qj_fill_map(MapParams* m, int n_top, const double* top_roots, const double* 
   // The fixed-point roots share one exponent, that of the largest within
   // 2^3 of the median root, so that a difference needs no shifts; larger
   // roots keep their own.
-  if (!top_exp.empty()) {
-    std::vector<int> sorted(top_exp);
-    std::sort(sorted.begin(), sorted.end());
-    const int most = sorted[sorted.size() / 2] + 3;
-    m->afx = *(std::upper_bound(sorted.begin(), sorted.end(), most) - 1);
+  const int n = n_top + n_bot;
+  if (n > 0) {
+    std::sort(sorted, sorted + n);
+    m->afx = *(std::upper_bound(sorted, sorted + n, sorted[n / 2] + 3) - 1);
   }
-  for (int i = 0; i < n_top + n_bot; i++) {
+  for (int i = 0; i < n; i++) {
     const double* r = m->r64[i];
     const fx_quat fq = fx_quat_at(r[0], r[1], r[2], r[3], std::max(m->afx, top_exp[i]));
     m->rfx[i][0] = fq.w;
