@@ -23,11 +23,12 @@ int qjg_set_timing(qjg_ctx* ctx, int on);
  * (synchronizes with it); a kernel that did not run reports 0. */
 int qjg_last_timings(qjg_ctx* ctx, float* ms_bulk, float* ms_refine);
 
-/* Map applications the FP32 bulk passes of this context carried out, summed
- * over the field calls whose counters were read (qjg_field_stats_read, the
- * host field and the streaming mesher read them; each read adds its call's).  qjg_field_stats.voxel_iters
- * counts orbit lengths: it is larger, because an orbit that repeats is not
- * applied to its end. */
+/* Map applications that the FP32 bulk pass of one call carried out: the call
+ * whose counters were read last (by qjg_field_stats_read; by the host field,
+ * the streaming mesher and qjg_mesh_async_result, of all their slabs).  0 for
+ * the FP64 form, which has no bulk pass.  qjg_field_stats.voxel_iters counts
+ * orbit lengths: it is larger, because an orbit that repeats is not applied to
+ * its end. */
 int64_t qjg_field_applied(qjg_ctx* ctx);
 
 /* Kernels this context has launched since it was created. */

@@ -61,11 +61,10 @@ def bench_mesh(args):
         raise SystemExit("raise --vert-cap/--tri-cap: needs %d / %d" % (st["n_verts"], st["n_tris"]))
     torch.cuda.synchronize()
     t0 = time.perf_counter()
-    before = ctx.field_applied()
     _, st = ctx.mesh_stream(h, g, it, **kw)
     torch.cuda.synchronize()
     wall = time.perf_counter() - t0
-    applied = ctx.field_applied() - before
+    applied = ctx.field_applied()
     # the field alone over the same grid, for the split
     f = torch.empty(g.res[0] * g.res[1] * min(g.res[2], args.slab + 1), dtype=torch.float64,
                     device="cuda")
@@ -620,10 +619,9 @@ def bench_large(args):
         e0, e1 = _events(torch)
         t0 = time.perf_counter()
         e0.record()
-        before = ctx.field_applied()
         rc, st = ctx.mesh_stream(h, g, it, check=False, d_verts32=v32.data_ptr(), vert_cap=vcap,
                                  d_tris=tris.data_ptr(), tri_cap=tcap, slab_nz=args.slab)
-        applied = ctx.field_applied() - before
+        applied = ctx.field_applied()
         e1.record()
         torch.cuda.synchronize()
         wall = time.perf_counter() - t0
@@ -668,7 +666,7 @@ def bench_large(args):
         buf = torch.empty(args.slab * XY, dtype=torch.float64, device="cuda")
         bulk = rest = 0.0
         tot = {}
-        before = ctx.field_applied()
+        applied = 0
         for z0 in range(0, g.res[2], args.slab):
             z1 = min(z0 + args.slab, g.res[2])
             ctx.field(h, g, it, buf.data_ptr(), z0=z0, z1=z1)
@@ -676,8 +674,8 @@ def bench_large(args):
             bulk, rest = bulk + b, rest + r
             for k, v in ctx.stats().items():
                 tot[k] = tot.get(k, 0) + v
+            applied += ctx.field_applied()
         del buf
-        applied = ctx.field_applied() - before
         flops = field_flops(rs, applied)
         field_gvox = n / ((bulk + rest) * 1e-3) / 1e9
         out["field_alone"] = {

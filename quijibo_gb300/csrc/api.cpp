@@ -391,7 +391,7 @@ int qjg_field_stats_read(qjg_ctx* ctx, void* stream, qjg_field_stats* out) {
   out->lane_iters = (int64_t)st.aux[3];
   out->rerun = (int64_t)st.rerun;
   out->rerun_iters = (int64_t)st.rerun_iters;
-  ctx->applied += (int64_t)st.applied;
+  ctx->applied = (int64_t)st.applied;
   return QJG_OK;
 }
 
@@ -460,6 +460,7 @@ int qjg_field_host(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg
   QJ_CUDA(ctx, cudaStreamSynchronize(cs));
   QJ_CUDA(ctx, cudaStreamSynchronize(xs));
   qjg_field_stats total = {};
+  ctx->applied = 0;
   const int roots = ctx->last_roots;
   for (int64_t k = 0; k < n_chunks; k++) {
     const DevStats& st = ctx->h_stats[k];

@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(128) field32_kernel(const __grid_constant__ Ma
     warp_append(route == TO_FF, (uint32_t)i, 0, false, 0, 0, &st->rerun, rl.ff, nullptr);
   }
   warp_add(&st->voxel_iters, iters_acc);
+  warp_add(&st->applied, iters_acc);  // every orbit is applied to its end
   warp_add(&st->nonfinite, nonfinite_acc);
   warp_add(&st->aux[3], lane_iters_acc);
 }

@@ -148,6 +148,7 @@ int mesh_core(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg_iter
   const long long S = (X + 63) / 64;  // units per row (qj::mesh_units)
 
   long long nv = 0, nt = 0;
+  int64_t applied = 0;  // qjg_field_applied of the slabs
   long long n_carry = 0, prev_nc = 0;  // cube entries carried into the slab; the last slab's count
   int cur = 0;                         // cube list of this slab (the other takes the carry)
   int prevL = 0;
@@ -182,6 +183,7 @@ int mesh_core(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg_iter
           return rc;
       }
       if ((rc = qjg_field_stats_read(ctx, s, &fs))) return rc;
+      applied += ctx->applied;
       if (timed) {
         float ms_bulk = 0.f, ms_rest = 0.f;
         if ((rc = qjg_last_timings(ctx, &ms_bulk, &ms_rest))) return rc;
@@ -313,6 +315,7 @@ int mesh_core(qjg_ctx* ctx, qjg_rootset rs, const qjg_grid* grid, const qjg_iter
     QJ_CUDA(ctx, cudaStreamSynchronize(s));
     nt += nt_last;
   }
+  if (streaming) ctx->applied = applied;
   // the parked edges of every slab, resolved together
   const bool any_parked = iter && iter->precision != QJG_FP64 && bisect && nv > 0;
   if (any_parked) {
@@ -616,7 +619,7 @@ int qjg_mesh_async_result(qjg_ctx* ctx, qjg_mesh_stats* stats) {
   st.field.lane_iters = (int64_t)fs.aux[3];
   st.field.rerun = (int64_t)fs.rerun;
   st.field.rerun_iters = (int64_t)fs.rerun_iters;
-  ctx->applied += (int64_t)fs.applied;
+  ctx->applied = (int64_t)fs.applied;
   *stats = st;
   if (run.overflow)
     return fail(ctx, QJG_ERR_CAPACITY, "the mesh outgrew the capacities of the fixed sequence");

@@ -42,7 +42,7 @@ struct qjg_ctx {
   // bookkeeping of the last field call, for qjg_field_stats_read
   int64_t last_voxels = 0;
   int last_roots = 0;
-  int64_t applied = 0;  // bulk-pass map applications of the calls whose counters were read
+  int64_t applied = 0;  // bulk-pass map applications of the call whose counters were read last
   // measurement hooks
   bool timing = false;
   bool timed_refine = false;

@@ -659,7 +659,8 @@ class Context:
         return a.value, b.value
 
     def field_applied(self):
-        """Map applications the FP32 bulk passes carried out so far."""
+        """Map applications the FP32 bulk pass carried out, of the call whose
+        counters were read last (stats(), field_host(), mesh_stream())."""
         return int(self.L.qjg_field_applied(self.h))
 
     def launch_count(self):
