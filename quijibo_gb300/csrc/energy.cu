@@ -143,18 +143,10 @@ __device__ __forceinline__ QX xpow(const Q& q, double e) {
   return xnorm(Q{mul(em, c), mul(scale2, q.x), mul(scale2, q.y), mul(scale2, q.z)}, (int)k);
 }
 
-__device__ __forceinline__ QX xpow_int(const Q& d, int n) {
-  const QX b = xof(d);
-  QX r = b;
-  for (int k = 1; k < n; k++) r = xmul(r, b);
-  return r;
-}
-
 // The map iterated in extended range from q0 (an FP64 overflow detected):
 // returns log|q_N| (0 where it is still not a number, as the reference's
 // stillNans); the last application's factors go to (Pf, Pe) and its top and
 // bottom products to *T, *B.
-template <bool POW_REF>
 __device__ __noinline__ double ext_map(const MapParams& m, const Q q0, int max_it, Q* Pf, int* Pe,
                                        QX* Tout, QX* Bout) {
   const int nt = m.nt, nb = m.nb;
@@ -171,7 +163,7 @@ __device__ __noinline__ double ext_map(const MapParams& m, const Q q0, int max_i
       for (int i = lo; i < hi; i++) {
         const Q d{sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
                   sub(q.z, m.r64[i][3])};
-        const QX f = POW_REF ? xpow(d, m.e64[i]) : xpow_int(d, m.ie[i]);
+        const QX f = xpow(d, m.e64[i]);
         Pf[i] = f.m;
         Pe[i] = f.e;
         acc = (i == lo) ? f : xmul(acc, f);
@@ -213,7 +205,7 @@ struct Voxel {
   bool bases_ok;
 };
 
-template <bool POW_REF, bool BOUNDS>
+template <bool BOUNDS>
 __device__ __forceinline__ void eval_voxel(const MapParams& m, const Q& q0, int max_it, Q* Pf,
                                            Q* Sf, Voxel& v) {
   const int nt = m.nt, nb = m.nb;
@@ -242,7 +234,7 @@ __device__ __forceinline__ void eval_voxel(const MapParams& m, const Q& q0, int 
         for (int i = lo; i < hi; i++) {
           const Q d{sub(q.w, m.r64[i][0]), sub(q.x, m.r64[i][1]), sub(q.y, m.r64[i][2]),
                     sub(q.z, m.r64[i][3])};
-          Pf[i] = POW_REF ? qpow(d, m.e64[i]) : qpow_int(d, m.ie[i]);
+          Pf[i] = qpow(d, m.e64[i]);
           acc_q = (i == lo) ? Pf[i] : qmul(acc_q, Pf[i]);
           if (BOUNDS) {
             v.spread += abs(ilog2_bits(norm2(Pf[i])));
@@ -306,7 +298,6 @@ __device__ __forceinline__ bool grad_setup(const Voxel& v, double logs, double a
 
 // The per-parameter gradient terms of one voxel (FP64 path) and their warp
 // sums; every lane of the warp calls it (inactive lanes with ok = false).
-template <bool POW_REF>
 __device__ __forceinline__ void grad_terms(const MapParams& m, const Voxel& v, bool ok,
                                            const Q& R, double dSdF, double RR, const Q* Pf,
                                            const Q* Sf, double* acc, int s_bad) {
@@ -315,7 +306,7 @@ __device__ __forceinline__ void grad_terms(const MapParams& m, const Voxel& v, b
   const Q& T = v.T;
   const Q& B = v.B;
   // one application from q0: the map's factor is the gradient's power, bit for bit
-  const bool reuse = POW_REF && v.its == 1;
+  const bool reuse = v.its == 1;
   // x / B = x * (conj(B) / |B|^2) (operator/): B's factor once, not per term
   Q Bi = {0, 0, 0, 0};
   if (ok) {
@@ -674,7 +665,7 @@ __global__ void __launch_bounds__(32, 16) tanh_grad_kernel(const __grid_constant
         }
       }
     }
-    grad_terms<true>(m, v, general, R, dSdF, RR, Pf, Sf, acc, s_bad);
+    grad_terms(m, v, general, R, dSdF, RR, Pf, Sf, acc, s_bad);
   };
   // the queued voxels' terms: each lane re-evaluates one voxel's map
   auto drain = [&](int count) {
@@ -688,7 +679,7 @@ __global__ void __launch_bounds__(32, 16) tanh_grad_kernel(const __grid_constant
       cell(queue[lane], p);
       const Q q0{p[0], p[1], p[2], g.slice};
       if (ONE) eval_one(m, q0, Pf, Lg, Sf, v);
-      else eval_voxel<true, false>(m, q0, max_it, Pf, Sf, v);
+      else eval_voxel<false>(m, q0, max_it, Pf, Sf, v);
       good = grad_setup(v, logs, alpha, thr, trilinear(wg, weights, p), R, dSdF, RR);
     } else {
       v.its = 0;
@@ -713,10 +704,10 @@ __global__ void __launch_bounds__(32, 16) tanh_grad_kernel(const __grid_constant
       cell(idx, p);
       q0 = Q{p[0], p[1], p[2], g.slice};
       if (ONE) eval_one(m, q0, Pf, Lg, Sf, v);
-      else eval_voxel<true, true>(m, q0, max_it, Pf, Sf, v);
+      else eval_voxel<true>(m, q0, max_it, Pf, Sf, v);
       double fval = 0.0;
       if (v.iterated || v.mg >= 1e-8) fval = log(v.mg);
-      if (!(mag(q0) < 1e-8) && v.over) fval = ext_map<true>(m, q0, max_it, Pf, Pe, &Tx, &Bx);
+      if (!(mag(q0) < 1e-8) && v.over) fval = ext_map(m, q0, max_it, Pf, Pe, &Tx, &Bx);
       if (field) field[idx] = fval;
       const double w = trilinear(wg, weights, p);
       const double S0 = tanh(mul(alpha, fval));
