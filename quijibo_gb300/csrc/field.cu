@@ -304,12 +304,18 @@ struct BulkAcc {
 // before (period 1) and with a marked one up to ORBIT_WINDOW steps back, and
 // on a match takes the remaining steps' |q|^2 and |grad log|R||^2 from the
 // last period instead of applying the map.  The results have the bits of the
-// full loop; maps whose orbits do not settle pay about 20 of ~950 issue
-// slots per application (16 / 8 roots) for the comparisons.  Measured, whole
-// qjg_field calls of the precision form: 512^3, 16 / 8 roots, 40 iterations
-// 91.5 -> 44.3 ms; 2200 x 2200 x 4, 48 / 24 roots, 60 iterations 83.3 -> 21.8
-// ms; 203 x 171 x 139, 23 / 11 roots, 30 iterations with the distance
-// estimate 9.7 -> 5.2 ms.
+// full loop.  Equal iterates have equal |q|^2, so only where a lane of the
+// warp finds |q|^2 again does the warp compare the rest (the bulk pass's
+// lanes stay together for it): 512^3 37.5 -> 36.2 ms against comparing all of
+// q at every step.  Measured, whole qjg_field calls of the precision form,
+// against the loop without the watch: 512^3, 16 / 8 roots, 40 iterations 91.5
+// -> 44.3 ms; 2200 x 2200 x 4, 48 / 24 roots, 60 iterations 83.3 -> 21.8 ms;
+// 203 x 171 x 139, 23 / 11 roots, 30 iterations with the distance estimate
+// 9.7 -> 5.2 ms.  Where no orbit settles before the cap (256^3, 12 iterations)
+// a call takes 0.93 of that loop's time with the distance estimate and 1.04
+// without at 16 / 8 roots, 0.99 and 1.03 at 8 / 0; caps too short to settle
+// in take the loop without the watch (launch_field32).
+//
 // A thread's marked iterates and the steps since, in shared memory (a
 // register copy would cost the unrolled kernels a resident block).
 struct OrbitLog {
@@ -365,8 +371,9 @@ __device__ __forceinline__ void orbit_replay(Orbit32& o, int period, const Orbit
 }
 
 // Runs the orbits of a lane's two voxels from q to their ends; returns the
-// map applications the lane's loop took.
-template <bool DE, int NT, int NB>
+// map applications the loop took.  WATCH: with the watch for repeats; WARP:
+// the whole warp is here and stays together.
+template <bool DE, int NT, int NB, bool WATCH = true, bool WARP = true>
 __device__ __forceinline__ int run_orbits(const MapParams& m, q32x2::Q2& q, Orbit32& a, Orbit32& b,
                                           float esc2, int max_it, OrbitLog& log,
                                           unsigned long long& applied) {
@@ -378,28 +385,46 @@ __device__ __forceinline__ int run_orbits(const MapParams& m, q32x2::Q2& q, Orbi
   };
   const int n0 = a.n + b.n;
   int step = 0, since = 0, pa = 0, pb = 0;
+  if (!WATCH) {
+    while (a.live || b.live) {
+      float2 gg = pair(0.f);
+      q = apply32x2<DE, NT, NB, true>(m, q, &gg);
+      const float2 m2 = norm2(q);
+      orbit_step<DE>(a, m2.x, gg.x, esc2, max_it);
+      orbit_step<DE>(b, m2.y, gg.y, esc2, max_it);
+      step++;
+    }
+    applied += a.n + b.n - n0;
+    return step;
+  }
+  float2 mark2 = norm2(q);
   set_mark();
-  while (a.live || b.live) {
+  while (WARP ? __any_sync(0xffffffffu, a.live || b.live) : a.live || b.live) {
     const Q2 p = q;
     float2 gg = pair(0.f);
     q = apply32x2<DE, NT, NB>(m, q, &gg);
     const float2 m2 = norm2(q);
+    const bool ea = a.live && (same_bits(m2.x, a.m2) || same_bits(m2.x, mark2.x));
+    const bool eb = b.live && (same_bits(m2.y, b.m2) || same_bits(m2.y, mark2.y));
     if (a.live) log.step[0][since][tid] = make_float2(m2.x, gg.x);
     if (b.live) log.step[1][since][tid] = make_float2(m2.y, gg.y);
     orbit_step<DE>(a, m2.x, gg.x, esc2, max_it);
     orbit_step<DE>(b, m2.y, gg.y, esc2, max_it);
     step++;
     since++;
-    if (a.live && (pa = orbit_period(lo(q), lo(p), log.mark[0][tid], since))) {
-      if (pa == 1) log.step[0][0][tid] = make_float2(m2.x, gg.x);
-      a.live = false;
-    }
-    if (b.live && (pb = orbit_period(hi(q), hi(p), log.mark[1][tid], since))) {
-      if (pb == 1) log.step[1][0][tid] = make_float2(m2.y, gg.y);
-      b.live = false;
+    if (WARP ? __any_sync(0xffffffffu, ea || eb) : ea || eb) {
+      if (ea && a.live && (pa = orbit_period(lo(q), lo(p), log.mark[0][tid], since))) {
+        if (pa == 1) log.step[0][0][tid] = make_float2(m2.x, gg.x);
+        a.live = false;
+      }
+      if (eb && b.live && (pb = orbit_period(hi(q), hi(p), log.mark[1][tid], since))) {
+        if (pb == 1) log.step[1][0][tid] = make_float2(m2.y, gg.y);
+        b.live = false;
+      }
     }
     if (since == mark_gap(step)) {
       set_mark();
+      mark2 = m2;
       since = 0;
     }
   }
@@ -412,7 +437,7 @@ __device__ __forceinline__ int run_orbits(const MapParams& m, q32x2::Q2& q, Orbi
 // One 16 x 4 tile (tile index t of the launch's z-range) of the two-voxel
 // bulk pass; list entries are `tag | local voxel index`.  Returns the
 // executed map applications of the warp's voxels (summed over the warp).
-template <bool DE, int NT = 0, int NB = 0>
+template <bool DE, int NT = 0, int NB = 0, bool WATCH = true>
 __device__ __forceinline__ unsigned long long tile2(const MapParams& m, const GridParams& g,
                                                     const IterParams& it, long long t,
                                                     double* __restrict__ field,
@@ -435,7 +460,7 @@ __device__ __forceinline__ unsigned long long tile2(const MapParams& m, const Gr
   const float2 m20 = norm2(q);
   Orbit32 a = orbit_start(va, m20.x, esc2, it.max_it);
   Orbit32 b = orbit_start(vb, m20.y, esc2, it.max_it);
-  const int steps = run_orbits<DE, NT, NB>(m, q, a, b, esc2, it.max_it, log, acc.applied);
+  const int steps = run_orbits<DE, NT, NB, WATCH>(m, q, a, b, esc2, it.max_it, log, acc.applied);
   acc.iters += a.n + b.n;
   const long long i = ((long long)zl * g.Y + y) * g.X + x;
   const int ra = va ? orbit_finish<DE>(a, it, esc2, l2band, refine, allow_ff, i, field, de,
@@ -455,10 +480,11 @@ __device__ __forceinline__ unsigned long long tile2(const MapParams& m, const Gr
 }
 
 // The forms with compiled-in counts (NT > 0) ask for 4 resident blocks per SM
-// (5: 512^3 at 16 / 8 roots 34.9 -> 35.9 ms; the looped form is unchanged by
-// it).
-template <bool DE, int NT = 0, int NB = 0>
-__global__ void __launch_bounds__(128, NT > 0 ? 4 : 0) field32x2_kernel(const __grid_constant__ MapParams m,
+// with the distance estimate (5: 512^3 at 16 / 8 roots 34.9 -> 35.9 ms), 5
+// without (256^3 at 16 / 8, 12 iterations: 2.34 -> 2.29 ms); the looped form is
+// unchanged by it.
+template <bool DE, int NT, int NB, bool WATCH>
+__global__ void __launch_bounds__(128, NT == 0 ? 0 : DE ? 4 : 5) field32x2_kernel(const __grid_constant__ MapParams m,
                                                         const GridParams g, const IterParams it,
                                                         double* __restrict__ field,
                                                         float* __restrict__ de, RefineLists rl,
@@ -471,7 +497,7 @@ __global__ void __launch_bounds__(128, NT > 0 ? 4 : 0) field32x2_kernel(const __
   for (;;) {
     const long long t = next_tile(&st->tiles_done);
     if (t >= tm.total) break;
-    tile2<DE, NT, NB>(m, g, it, t, field, de, rl, refine, allow_ff, 0u, st, acc, esc2, l2band, log);
+    tile2<DE, NT, NB, WATCH>(m, g, it, t, field, de, rl, refine, allow_ff, 0u, st, acc, esc2, l2band, log);
   }
   warp_add(&st->voxel_iters, acc.iters);
   warp_add(&st->applied, acc.applied);
@@ -544,7 +570,7 @@ __device__ __forceinline__ void rerun_pair(const MapParams& m, const GridParams&
   ob->err = q32::EPS32;
   q32x2::Q2 qf = qff2::hi(q);
   unsigned long long applied = 0;
-  run_orbits<true, 0, 0>(m, qf, *oa, *ob, esc2, it.max_it, log, applied);
+  run_orbits<true, 0, 0, true, false>(m, qf, *oa, *ob, esc2, it.max_it, log, applied);
   *ra = orbit_finish<true>(*oa, it, esc2, l2band, 1, false, ia, field, de, nonfinite_acc);
   *rb = vb ? orbit_finish<true>(*ob, it, esc2, l2band, 1, false, ib, field, de, nonfinite_acc)
            : WRITTEN;
@@ -751,15 +777,19 @@ cudaError_t launch_field32(const MapParams& m, const GridParams& g, const IterPa
     // root counts of the workloads' maps compiled in, two root pairs per trip
     // (4% faster at 16 / 8 and at 48 / 24 roots than the kernel that reads
     // its counts, which also ran 4% slower with two pairs per trip)
-#define QJ_F32X2(NT, NB)                                                                   \
-  do {                                                                                     \
-    const void* fn = want ? (const void*)field32x2_kernel<true, NT, NB>                   \
-                          : (const void*)field32x2_kernel<false, NT, NB>;                 \
-    const int blocks = grid_blocks(fn, 128);                                               \
-    if (want)                                                                              \
-      field32x2_kernel<true, NT, NB><<<blocks, 128, 0, s>>>(m, g, it, field, de, rl, r, st); \
-    else                                                                                   \
-      field32x2_kernel<false, NT, NB><<<blocks, 128, 0, s>>>(m, g, it, field, de, rl, 0, st); \
+    //
+    // Orbits that settle do so after 5-15 applications, those of maps with
+    // many roots first.  With a cap of 8 the watch costs 11% at 16 / 8 roots
+    // and 12% at 8 / 0 and finds little, and saves 20-30% at 48 / 24; with one
+    // of 12 it saves 10-35% at 12 / 4 roots.
+    const bool watch = it.max_it >= (m.nt + m.nb >= 32 ? 6 : 9);
+#define QJ_F32X2(NT, NB)                                                              \
+  do {                                                                                \
+    const auto fn = want ? watch ? field32x2_kernel<true, NT, NB, true>               \
+                                 : field32x2_kernel<true, NT, NB, false>              \
+                    : watch ? field32x2_kernel<false, NT, NB, true>                   \
+                            : field32x2_kernel<false, NT, NB, false>;                 \
+    fn<<<grid_blocks((const void*)fn, 128), 128, 0, s>>>(m, g, it, field, de, rl, r, st); \
   } while (0)
     if (m.lagrange)
       QJ_F32X2(0, 0);

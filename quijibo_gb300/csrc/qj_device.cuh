@@ -877,13 +877,17 @@ __device__ __forceinline__ q32x2::Q2 product32x2(const MapParams& m, const q32x2
 // stalled per issue) once settled orbits left the loop after about ten
 // trips: 512^3 at 16 / 8 roots 40.3 ms whole call unrolled, 36.7 at three
 // pairs per trip, 34.9 at two, 35.4 at one; 2200 x 2200 x 4 at 48 / 24 roots
-// 11.4 (24 unrolled), 10.7, 10.6, 10.7.
-template <bool DE, int LO, int N>
+// 11.4 (24 unrolled), 10.7, 10.6, 10.7.  Unrolled all the same: a map of eight
+// top roots and no bottom ones (320^3, 8 iterations, nothing settled: 1.54 ->
+// 1.20 ms), eight roots without the distance estimate (256^3 at 16 / 8, 8
+// iterations 1.73 -> 1.66 ms), and up to 24 of these in the loop that watches
+// for no repeat (1.49 ms; FULL).
+template <bool DE, int LO, int N, bool FULL>
 __device__ __forceinline__ q32x2::Q2 product32x2_fixed(const MapParams& m, const q32x2::Q2& q,
                                                        q32x2::Q2& g) {
   using namespace q32x2;
   Q2 r = root_term32x2<DE>(m, q, LO, g);
-#pragma unroll 2
+#pragma unroll (FULL && !DE && N <= 24) || (N <= 8 && (LO == 0 || !DE)) ? 12 : 2
   for (int k = 1; k + 1 < N; k += 2) {
     const Q2 t0 = root_term32x2<DE>(m, q, LO + k, g);
     const Q2 t1 = root_term32x2<DE>(m, q, LO + k + 1, g);
@@ -923,7 +927,7 @@ __device__ __forceinline__ q32x2::Q2 lagrange32x2(const MapParams& m, const q32x
 
 // NT, NB > 0: the root counts are compile-time constants (they must equal
 // m.nt and m.nb; the quotient order only); 0: read from m.
-template <bool DE, int NT = 0, int NB = 0>
+template <bool DE, int NT = 0, int NB = 0, bool FULL = false>
 __device__ __forceinline__ q32x2::Q2 apply32x2(const MapParams& m, const q32x2::Q2& q,
                                                float2* g2) {
   using namespace q32x2;
@@ -938,11 +942,11 @@ __device__ __forceinline__ q32x2::Q2 apply32x2(const MapParams& m, const q32x2::
     if (DE) *g2 = norm2(g);
     return out;
   }
-  const Q2 top = NT > 0 ? product32x2_fixed<DE, 0, (NT > 0 ? NT : 1)>(m, q, g)
+  const Q2 top = NT > 0 ? product32x2_fixed<DE, 0, (NT > 0 ? NT : 1), FULL>(m, q, g)
                         : product32x2<DE>(m, q, 0, m.nt, g);
   Q2 out;
   if (NT > 0 ? NB > 0 : m.nb > 0) {
-    const Q2 bot = NT > 0 ? product32x2_fixed<DE, (NT > 0 ? NT : 0), (NB > 0 ? NB : 1)>(m, q, g)
+    const Q2 bot = NT > 0 ? product32x2_fixed<DE, (NT > 0 ? NT : 0), (NB > 0 ? NB : 1), FULL>(m, q, g)
                           : product32x2<DE>(m, q, m.nt, m.nt + m.nb, g);
     const float2 n = norm2(bot);
     const float2 inv =

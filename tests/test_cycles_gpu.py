@@ -202,3 +202,30 @@ def test_fp32_gradient_on_cycles(ctx, p, rate, max_it):
     for e, g in zip(es, grads):
         assert abs(e - e32) <= 1e-6 * abs(e32)
         assert np.linalg.norm(g.cpu().numpy() - g32) <= 1e-5 * np.linalg.norm(g32)
+
+
+# --------------------------------------- caps about the line of the watch
+
+@pytest.mark.parametrize("max_it", [5, 6, 8, 9])
+@pytest.mark.parametrize("nt,nb", [(8, 0), (16, 8), (48, 24), (24, 8), (23, 8)])
+@pytest.mark.parametrize("de", [False, True])
+def test_caps_about_the_watch(ctx, nt, nb, max_it, de):
+    """Below 9 applications (6 with 32 roots or more) nothing is watched:
+    every orbit is applied to its end, with the same values."""
+    h, g = ctx.upload(settling_map(nt, nt, nb)), Grid((35, 22, 5))
+    it = ctx.iter_params(max_it, 2.0, precision=lib.QJG_FP32, want_de=de)
+    out = []
+    try:
+        for pairs in (True, False):
+            lib.set_field32_pairs(pairs)
+            out.append((*ctx.field_host(h, g, it, de=de), ctx.field_applied()))
+    finally:
+        lib.set_field32_pairs(True)
+        ctx.free(h)
+    (fa, da, sa, na), (fb, db, sb, _) = out
+    assert np.array_equal(fa.view(np.uint64), fb.view(np.uint64))
+    if de:
+        assert np.array_equal(da.view(np.uint32), db.view(np.uint32))
+    assert sa["voxel_iters"] == sb["voxel_iters"] >= na
+    if max_it < (6 if nt + nb >= 32 else 9):
+        assert na == sa["voxel_iters"]
