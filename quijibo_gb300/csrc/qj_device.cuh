@@ -484,10 +484,11 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
 // order: plain FP64 field 64^3 6.7 -> 4.5 ms, FP64 mesh 48^3 9.2 -> 6.1 ms
 // (12 / 6 roots; 5.3 and 6.9 ms with a loop for each side and the FP64 chain
 // expanded in place: the code has to stay small for instruction fetch).  The
-// tests and the cut of magnitudes cost what the roots' common exponent and
-// the division in fixed point give back where the pipes are full (one refine
-// pass 5.17 -> 5.03 ms, FP64 15%, ALU 56% busy), and 5-10% where one warp's
-// chain is waited for (32^3 field 353 -> 372 us).  The product of 24 factors
+// tests and the cut of magnitudes cost less than the roots' common exponent,
+// the division in fixed point and a 32-bit count of leading zeros give back
+// where the pipes are full (a mesh of such a grid, whole call, 29.8 -> 27.5 ms
+// against floors of products and no tests), and 4-10% where one warp's chain
+// is waited for (32^3 field 350 -> 365 us).  The product of 24 factors
 // is off by 0.55 units of 2^-53 (rms), the fused one by 3.8.
 template <int POW_REF, bool DE>
 __device__ __forceinline__ q64::Q quotient_fx(const MapParams& m, const q64::Q& q, q64::Q& g,

@@ -428,10 +428,17 @@ FX_FN fx_quat fx_joined(fx_quat q) {
   q.z = fx_signed(q.mz, q.sz);
   return q;
 }
-// The largest magnitude's top bit to 2^61; none is 2^62 or more.
+FX_FN int fx_clz32(uint32_t a) {
+#ifdef __CUDACC__
+  return __clz((int)a);
+#else
+  return a ? __builtin_clz(a) : 32;
+#endif
+}
+// The largest magnitude's top bit to 2^61; none is 2^62 or more, and one has
+// a high half (or all are zero: so they stay).
 FX_FN fx_quat fx_norm(fx_quat q) {
-  const fx_u64 any = q.mw | q.mx | q.my | q.mz;
-  const int s = any ? fx_clz(any) - 2 : 61;
+  const int s = fx_clz32(fx_high(q.mw) | fx_high(q.mx) | fx_high(q.my) | fx_high(q.mz)) - 2;
   q.mw <<= s;
   q.mx <<= s;
   q.my <<= s;
@@ -506,9 +513,8 @@ FX_FN fx_quat fx_qsub(fx_quat a, fx_quat b) {
   o = fx_split(o);
   o.odd = (fx_high(o.mw) == 0) | (fx_high(o.mx) == 0) << 1 | (fx_high(o.my) == 0) << 2 |
           (fx_high(o.mz) == 0) << 3;
-  // below 2^63: the top bit to 2^62, then half
-  const fx_u64 any = o.mw | o.mx | o.my | o.mz;
-  const int s = any ? fx_clz(any) - 1 : 62;
+  // below 2^63: the top bit to 2^62, then half (no high half: fx_near)
+  const int s = fx_clz32(fx_high(o.mw) | fx_high(o.mx) | fx_high(o.my) | fx_high(o.mz)) - 1;
   o.mw = o.mw << s >> 1;
   o.mx = o.mx << s >> 1;
   o.my = o.my << s >> 1;
@@ -527,8 +533,8 @@ FX_FN fx_u64 fx_flip(fx_u64 m, int32_t s) { return m ^ fx_mask(s); }
 FX_FN fx_i64 fx_sum4(fx_u64 a1, fx_u64 b1, int32_t s1, fx_u64 a2, fx_u64 b2, int32_t s2, fx_u64 a3,
                      fx_u64 b3, int32_t s3, fx_u64 a4, fx_u64 b4, int32_t s4) {
   const uint32_t minus = (uint32_t)-(s1 + s2 + s3 + s4);
-  return (fx_i64)(fx_flip(fx_mulhi(a1, b1), s1) + fx_flip(fx_mulhi(a2, b2), s2) +
-                  fx_flip(fx_mulhi(a3, b3), s3) + fx_flip(fx_mulhi(a4, b4), s4) + minus);
+  return (fx_i64)((fx_flip(fx_mulhi(a1, b1), s1) + fx_flip(fx_mulhi(a2, b2), s2) + minus) +
+                  (fx_flip(fx_mulhi(a3, b3), s3) + fx_flip(fx_mulhi(a4, b4), s4)));
 }
 // Whether all four terms are below 2^51 of at most 2^60 (by the high halves)
 // and not all zero.
