@@ -187,6 +187,7 @@ int qj_fill_map(MapParams* m, int n_top, const double* top_roots, const double* 
   if (n > 0) {
     std::sort(sorted, sorted + n);
     m->afx = *(std::upper_bound(sorted, sorted + n, sorted[n / 2] + 3) - 1);
+    m->beside = fx_beside_of(m->r64, n, m->afx);
   }
   for (int i = 0; i < n; i++) {
     const double* r = m->r64[i];

@@ -473,8 +473,8 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
 // or a partial product leaves [2^-500, 2^500], zero or not finite (its
 // overflow, underflow and NaN), or a component is small in all its terms or
 // the vector part as a whole, on and beside the real axis and coordinate
-// planes (fx_quat's odd; 2e-5 to 4e-4 of the applications over maps with
-// generic roots).  Without that test the orbits of q^3 + c left the real axis:
+// planes (fx_quat's odd, and fx_beside before any product; none of 10^6
+// applications of maps with generic roots).  Without that test the orbits of q^3 + c left the real axis:
 // 23 of 33 points on it had the other sign.
 // The FP64 pipe issues 1/64 of what the integer pipe does: as fused FP64
 // products the refine pass over a 128^3 grid whose inside needs it held that
@@ -490,13 +490,14 @@ __device__ __forceinline__ q64::Q product64(const MapParams& m, const q64::Q& q,
 // against floors of products and no tests), and 4-10% where one warp's chain
 // is waited for (32^3 field 350 -> 365 us).  The product of 24 factors
 // is off by 0.55 units of 2^-53 (rms), the fused one by 3.8.
+// top_exp: the larger exponent of q and the roots.
 template <int POW_REF, bool DE>
-__device__ __forceinline__ q64::Q quotient_fx(const MapParams& m, const q64::Q& q, q64::Q& g,
-                                              bool* odd) {
+__device__ __forceinline__ q64::Q quotient_fx(const MapParams& m, const q64::Q& q, int top_exp,
+                                              q64::Q& g, bool* odd) {
   using namespace q64;
   fx_quat qx, r, top;
   if (POW_REF == 0)
-    qx = fx_quat_at(q.w, q.x, q.y, q.z, max(m.afx, fx_top(q.w, q.x, q.y, q.z)));
+    qx = fx_quat_at(q.w, q.x, q.y, q.z, top_exp);
   const int nt = m.nt, n = nt + m.nb;
 #pragma unroll 1
   for (int i = 0; i < n; i++) {
@@ -610,8 +611,9 @@ __device__ __forceinline__ q64::Q apply64(const MapParams& m, const q64::Q& q, d
   } else if (POW_REF == 2) {
     out = quotient64<POW_REF, DE>(m, q, g);
   } else {
-    bool odd = false;
-    out = quotient_fx<POW_REF, DE>(m, q, g, &odd);
+    const int top = max(m.afx, fx_top(q.w, q.x, q.y, q.z));
+    bool odd = m.beside && fx_beside(m.beside, q.x, q.y, q.z, top);
+    if (!odd) out = quotient_fx<POW_REF, DE>(m, q, top, g, &odd);
     if (odd) {
       Q h;
       out = quotient64_far<POW_REF, DE>(m, q, &h);

@@ -377,9 +377,13 @@ FX_FN void fx_sincos(double x, double* sn, double* cs) {
 // quaternion, FP64's of each component.  Where a component is small in every
 // one of its terms (near the real axis or a coordinate plane with roots in
 // it), FP64 keeps it to 2^-53 of itself, and whether it is zero decides the
-// polar power's branch: `odd` then says that FP64's product is wanted, as
-// soon as all four terms of a component are below 2^-9 of the largest they
-// could be without all being zero, or the vector part as a whole is.
+// polar power's branch.  Maps with roots in such places are known when they
+// are uploaded (fx_beside); elsewhere `odd` says that FP64's product is
+// wanted, as soon as all four terms of a component are below 2^-16 of the
+// largest they could be without all being zero, or the vector part as a whole
+// is below 2^-20.  (At 2^-9, where fewer than 53 bits are left, a square's
+// small vector part met a small component of the product before it in 1e-3 of
+// a map's first applications, whose FP64 error is as large as ever.)
 typedef struct {
   fx_i64 w, x, y, z;       // the components, and as magnitude and sign (0 or
   fx_u64 mw, mx, my, mz;   // -1): the compiler drops what a caller leaves
@@ -536,13 +540,13 @@ FX_FN fx_i64 fx_sum4(fx_u64 a1, fx_u64 b1, int32_t s1, fx_u64 a2, fx_u64 b2, int
   return (fx_i64)((fx_flip(fx_mulhi(a1, b1), s1) + fx_flip(fx_mulhi(a2, b2), s2) + minus) +
                   (fx_flip(fx_mulhi(a3, b3), s3) + fx_flip(fx_mulhi(a4, b4), s4)));
 }
-// Whether all four terms are below 2^51 of at most 2^60 (by the high halves)
+// Whether all four terms are below 2^44 of at most 2^60 (by the high halves)
 // and not all zero.
 FX_FN int fx_lost(fx_u64 a1, fx_u64 b1, fx_u64 a2, fx_u64 b2, fx_u64 a3, fx_u64 b3, fx_u64 a4,
                   fx_u64 b4) {
   const fx_u64 most = (fx_u64)fx_high(a1) * fx_high(b1) | (fx_u64)fx_high(a2) * fx_high(b2) |
                       (fx_u64)fx_high(a3) * fx_high(b3) | (fx_u64)fx_high(a4) * fx_high(b4);
-  return most < (1ull << 51) && ((a1 && b1) || (a2 && b2) || (a3 && b3) || (a4 && b4));
+  return most < (1ull << 44) && ((a1 && b1) || (a2 && b2) || (a3 && b3) || (a4 && b4));
 }
 // The product; `strict`: of two factors of the map, odd as said above.
 FX_FN fx_quat fx_hamilton(fx_quat a, fx_quat b, int strict) {
@@ -560,11 +564,11 @@ FX_FN fx_quat fx_hamilton(fx_quat a, fx_quat b, int strict) {
   o = fx_norm(fx_split(o));
   if (strict) {
     // no small component on one side: its product with the other side's
-    // largest is a term of 2^51 or more in every component
+    // largest is a term of 2^44 or more in every component
     const uint32_t p = fx_least(fx_least(fx_high(a.mw), fx_high(a.mx)), fx_least(fx_high(a.my), fx_high(a.mz)));
     const uint32_t q = fx_least(fx_least(fx_high(b.mw), fx_high(b.mx)), fx_least(fx_high(b.my), fx_high(b.mz)));
-    const int real = fx_high(o.mx | o.my | o.mz) < (1u << 21);
-    if ((p < (1u << 22) && q < (1u << 22)) || real)
+    const int real = fx_high(o.mx | o.my | o.mz) < (1u << 10);
+    if ((p < (1u << 15) && q < (1u << 15)) || real)
       o.odd |= (real && ((a.mx | a.my | a.mz) || (b.mx | b.my | b.mz))) ||
                fx_lost(a.mw, b.mw, a.mx, b.mx, a.my, b.my, a.mz, b.mz) ||
                fx_lost(a.mw, b.mx, a.mx, b.mw, a.my, b.mz, a.mz, b.my) ||
@@ -584,6 +588,29 @@ FX_FN fx_quat fx_conj(fx_quat a) {
   a.sy = ~a.sy;
   a.sz = ~a.sz;
   return fx_joined(a);
+}
+// Maps whose roots all lie on the real axis or in a coordinate plane through
+// it, but for 2^-9 of their size: bits 0 to 2, components x to z small in
+// every root; bits 3 to 5, and not zero in all of them.  0 for other maps.
+FX_FN int fx_beside_of(const double (*r)[4], int n, int top) {
+  int small = 7, some = 0;
+  for (int i = 0; i < n; i++)
+    for (int c = 0; c < 3; c++) {
+      if (fx_field(r[i][c + 1]) >= top + 1022 - 9) small &= ~(1 << c);
+      if (r[i][c + 1] != 0.0) some |= 8 << c;
+    }
+  return small == 7 || small == 3 || small == 5 || small == 6 ? small | some : 0;
+}
+// Whether q lies beside that axis or plane: every difference q - root then has
+// those components below 2^-9 of its largest (top, the larger exponent of q
+// and the roots) and not zero.  A single plane needs both components off it
+// small; on the axis each counts, for all vector parts are q's multiples.
+FX_FN int fx_beside(int map, double x, double y, double z, int top) {
+  const int least = top + 1022 - 9;
+  const int s = (fx_field(x) < least) | (fx_field(y) < least) << 1 | (fx_field(z) < least) << 2;
+  const int some = (x != 0.0) | (y != 0.0) << 1 | (z != 0.0) << 2 | map >> 3;
+  const int small = map & 7, hit = s & some & small;
+  return hit && (small == 7 || (s & small) == small);
 }
 // v 2^k for a normal result, by the exponent field (0, infinities and NaN stay).
 FX_FN double fx_scale(double v, int k) {

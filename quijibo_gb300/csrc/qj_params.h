@@ -38,6 +38,7 @@ struct MapParams {
   alignas(16) long long rfx[QJ_MAX_ROOTS][4];
   int efx[QJ_MAX_ROOTS];
   int afx;
+  int beside;  // fx_beside_of the roots
   // the double-float head: each root coordinate and the scale as hi + lo
   alignas(8) float rff[QJ_MAX_ROOTS][4][2];
   float scale_ff[2];

@@ -26,6 +26,15 @@ void power(const double* q, long n, long long* o) {
   for (long i = 2; i < n; i++) r = fx_qpower(r, b);
   put(r, o);
 }
+void beside(const double* roots, const double* q, long n, long long* o) {
+  int top = -1100;
+  for (long i = 0; i < n; i++) {
+    const double* r = roots + 4 * i;
+    if (fx_top(r[0], r[1], r[2], r[3]) > top) top = fx_top(r[0], r[1], r[2], r[3]);
+  }
+  const int map = fx_beside_of((const double(*)[4])roots, (int)n, top), t = fx_top(q[0], q[1], q[2], q[3]);
+  o[5] = map && fx_beside(map, q[1], q[2], q[3], t > top ? t : top);
+}
 void difference(const double* a, const double* b, long long* o) { put(fx_qsub(get(a), get(b)), o); }
 """
 
@@ -97,7 +106,7 @@ def test_conjugate_factors_cancel(fx, kind):
 @pytest.mark.parametrize("kind", ["even", "scales", "plane", "axis", "twos"])
 def test_components_are_kept_or_marked(fx, kind):
     """A component's terms are cut by less than a unit each and its factors by
-    one before: 12 units.  Unmarked, the largest term has 2^51 of them."""
+    one before: 12 units.  Unmarked, the largest term has 2^44 of them."""
     rng = np.random.RandomState(3)
     marked = 0
     with mpmath.workprec(300):
@@ -114,7 +123,7 @@ def test_components_are_kept_or_marked(fx, kind):
                      [a[0] * b[3], a[1] * b[2], -a[2] * b[1], a[3] * b[0]]]
             for c in range(4):
                 got = mpmath.ldexp(int(v[c]), e - 62)
-                assert abs(got - sum(terms[c])) <= 12 * mpmath.mpf(2) ** -51 * max(abs(t) for t in terms[c])
+                assert abs(got - sum(terms[c])) <= 12 * mpmath.mpf(2) ** -44 * max(abs(t) for t in terms[c])
     assert marked <= 4 if kind == "even" else True
 
 
@@ -124,3 +133,21 @@ def test_a_tiny_component_is_marked(fx):
         assert fx("difference", [1.0, 0.5, tiny, 0.0], [0.25, 1.0, 0.0, 0.0])[2] & 4
     assert not fx("product", [[1.0, 0.0, 0.0, 0.0], [0.5, 0.0, 0.0, 0.0]], 2)[2]
     assert not fx("product", [[1.0, 0.5, 0.0, 0.0], [0.5, 0.25, 0.0, 0.0]], 2)[2]
+
+
+@pytest.mark.parametrize("roots,near,not_near", [
+    ("axis", [[1, 1e-3, 0.3, 0.3], [0.1, 1e-17, 0, 0], [2.0, 1e-3, 1e-3, 1e-3]],
+     [[1, 0, 0.3, 0.3], [1, 0, 0, 0], [1, 0.1, -0.1, 0.1]]),
+    ("plane", [[1, 0.3, 1e-3, 0], [0.2, 0.3, 1e-17, -1e-4]],
+     [[1, 0.3, 0, 0], [1, 0.3, 1e-3, 0.5], [1, 0, 0.1, 0.1]]),
+    ("almost", [[1, 0.3, 0, 0], [1, 0.3, 1e-3, 0]], [[1, 0.3, 0.2, 0.1]]),
+    ("flat", [], [[1, 0.3, 0.2, 0], [1, 0.3, 0.2, 1e-9], [1, 0, 0, 0]]),
+    ("any", [], [[1, 0.3, 1e-9, 0], [1, 1e-9, 1e-9, 1e-9]])])
+def test_beside_the_roots_axis_or_plane(fx, roots, near, not_near):
+    r = np.random.RandomState(4).uniform(-1.2, 1.2, (9, 4))
+    r[:, {"axis": slice(1, 4), "plane": slice(2, 4), "almost": slice(2, 4), "flat": slice(3, 4),
+          "any": slice(0, 0)}[roots]] *= 1e-6 if roots == "almost" else 0.0
+    for q in near:
+        assert fx("beside", r, q, 9)[2]
+    for q in not_near:
+        assert not fx("beside", r, q, 9)[2]
