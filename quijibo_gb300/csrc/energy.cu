@@ -1577,6 +1577,7 @@ __global__ void __launch_bounds__(SQF_T) sq_fwd2_kernel(
 // max_it - N so that long orbits come first: hist[bucket * nchunks + chunk].
 __global__ void __launch_bounds__(SQC_T) sq_chunk_kernel(const double* __restrict__ contrib,
                                                          const int* __restrict__ keys,
+                                                         const int* __restrict__ iters,
                                                          long long n, int max_it, int nchunks,
                                                          int* __restrict__ hist,
                                                          double* __restrict__ partials, int slots,
@@ -1588,11 +1589,12 @@ __global__ void __launch_bounds__(SQC_T) sq_chunk_kernel(const double* __restric
   for (int b = t; b <= max_it; b += SQC_T) h[b] = 0;
   __syncthreads();
   double e = 0.0, bad = 0.0;
-  unsigned long long steps = 0;  // orbit steps of the adjoint
+  unsigned long long steps = 0, lengths = 0;  // orbit steps of the adjoint; orbit lengths
   for (int i = t; i < SQ_CH; i += SQC_T) {
     const long long k = (long long)c * SQ_CH + i;
     if (k >= n) break;
     e += contrib[k];
+    lengths += (unsigned long long)iters[k];
     if (keys) {
       const int key = keys[k];
       if (key == -2) bad += 1.0;
@@ -1603,7 +1605,11 @@ __global__ void __launch_bounds__(SQC_T) sq_chunk_kernel(const double* __restric
     }
   }
   steps = __reduce_add_sync(0xffffffffu, (unsigned)steps);
-  if ((t & 31) == 0 && steps) atomicAdd(&work[1], steps);
+  lengths = __reduce_add_sync(0xffffffffu, (unsigned)lengths);
+  if ((t & 31) == 0 && (steps | lengths)) {
+    atomicAdd(&work[1], steps);
+    atomicAdd(&work[2], lengths);
+  }
   red_e[t] = e;
   red_b[t] = bad;
   __syncthreads();
@@ -2590,19 +2596,31 @@ __global__ void __launch_bounds__(32 * SQR_W) sq_reduce_item_kernel(
 
 // Forward kernel choice (qjg_set_energy_pairs): two samples per lane or one.
 std::atomic<int> g_sq_pairs{0};
-// Forward blocks per SM (qjg_set_energy_forward_blocks): 0 the rule in
-// sq_launch, else that many (capped by residency), for sweeps.
-// The forward grid's blocks per SM: three, more where a lane would get over
-// four samples.  A warp's lanes stay busy only while there are samples to
-// refill them, so more lanes pay only where nearly every orbit settles early
-// (us of an energy + gradient call at 3 / 4 / 5 / 8 blocks per SM, 200k
-// samples, 64/16 roots: 421 / 383 / 381 / 380; ms of a 50-step
-// L-BFGS fit of them, whose orbits spread more: 86 / 92 / 103 / 134).
-static long long sq_fwd_want(long long n, int sms) {
-  const long long lanes_per_sm = (long long)sms * SQF_T;
-  return std::max<long long>(3, ((n + 3) / 4 + lanes_per_sm - 1) / lanes_per_sm);
-}
+// Forward blocks per SM (qjg_set_energy_forward_blocks): 0 the rules below,
+// else that many (capped by residency), for sweeps.
 std::atomic<int> g_sq_fwd_blocks{0};
+
+static long long sq_blocks(long long lanes, int sms) {
+  const long long per_block = (long long)sms * SQF_T;
+  return std::max<long long>(3, (lanes + per_block - 1) / per_block);
+}
+// The forward grid's blocks per SM in FP64, which the FP64 pipe bounds: about
+// four samples a lane, at least three blocks.
+static long long sq_fwd_want64(long long n, int sms) { return sq_blocks((n + 3) / 4, sms); }
+// ... and in FP32, where the lane with the most orbit steps ends last and a
+// warp with one long orbit issues as much as one with 32.  `full` is the
+// call's orbit steps in full-length orbits: a lane for each, or for every
+// second, third, ... where they outnumber the lanes that can be resident (more
+// lanes would not end sooner, and cost issue slots).  Forward calls of 200k
+// samples, 30 iterations, ms at 3 / 5 / 6 / 8 blocks per SM: 64/16 roots, half
+// of the orbits at the cap 0.33 / 0.32 / 0.31 / 0.34 (the rule: 6); 8/4 roots,
+// 83% at it 0.32 / 0.28 / 0.29 / 0.32 (5); 64/16 fitted, 2% at it 0.53 / 0.70 /
+// 0.81 / 1.02 (3); 100k samples, 16/8, 96% 0.34 / 0.27 / 0.30 / 0.30 (5).
+static long long sq_fwd_want32(long long full, int sms, int per_sm) {
+  const long long most = (long long)sms * std::max(per_sm, 1) * SQF_T;
+  const long long rounds = std::max<long long>(1, (full + most - 1) / most);
+  return sq_blocks((full + rounds - 1) / rounds, sms);
+}
 
 // FP32 adjoint choice (qjg_set_energy_adjoint_roots): the roots of a step
 // spread over a group of lanes (sq_bwd_roots_kernel) or walked by one lane.
@@ -2630,7 +2648,7 @@ SqLayout sq_layout(bool fp64, bool grad, long long n, int max_it, int nt, int nb
   };
   const size_t nn = (size_t)std::max<long long>(n, 0);
   L.claim = take(sizeof(unsigned long long));
-  L.work = take(2 * sizeof(unsigned long long));
+  L.work = take(3 * sizeof(unsigned long long));
   L.total = take(sizeof(int));
   L.contrib = take(sizeof(double) * nn);
   L.keys = take(sizeof(int) * nn);
@@ -2677,7 +2695,7 @@ template <class T>
 cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const double* xyz,
                       const double* target, long long n, double slice, int max_it, double escape,
                       double d_sat, unsigned char* scr, const SqLayout& L, int* iters, int sms,
-                      cudaStream_t s, int* launches) {
+                      cudaStream_t s, int* launches, long long steps_hint) {
   const int nr = nt + nb;
   unsigned long long* claim = reinterpret_cast<unsigned long long*>(scr + L.claim);
   int* total = reinterpret_cast<int*>(scr + L.total);
@@ -2694,7 +2712,7 @@ cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const dou
     o.ck = reinterpret_cast<V4<T>*>(scr + L.ck);
   }
   cudaError_t e = cudaMemsetAsync(claim, 0, sizeof(unsigned long long), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, 3 * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
   const size_t sh_roots = sizeof(T) * 5 * nr;
   // persistent forward grid: as many blocks as stay resident
@@ -2705,7 +2723,12 @@ cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const dou
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sq_fwd_kernel<T, false>, SQF_T, sh_roots);
   if (e != cudaSuccess) return e;
   const int fixed = g_sq_fwd_blocks.load(std::memory_order_relaxed);
-  const long long want = fixed > 0 ? fixed : sq_fwd_want(n, sms);
+  // the steps of an earlier call on as many samples (steps_hint), else half
+  // the cap per sample
+  const long long full = steps_hint > 0 && max_it > 0 ? (steps_hint + max_it - 1) / max_it : (n + 1) / 2;
+  const long long want = fixed > 0                       ? fixed
+                         : std::is_same<T, float>::value ? sq_fwd_want32(full, sms, per_sm)
+                                                         : sq_fwd_want64(n, sms);
   const long long need = (n + SQF_T - 1) / SQF_T;
   const int fblocks = (int)std::max<long long>(
       1, std::min<long long>((long long)sms * std::min<long long>(std::max(per_sm, 1), want), need));
@@ -2724,7 +2747,7 @@ cudaError_t sq_launch(bool grad, const double* params, int nt, int nb, const dou
                                                              max_it, escape, d_sat, claim, o);
   }
   int* hist = grad ? reinterpret_cast<int*>(scr + L.hist) : nullptr;
-  sq_chunk_kernel<<<L.nchunks, SQC_T, 0, s>>>(o.contrib, grad ? o.keys : nullptr, n,
+  sq_chunk_kernel<<<L.nchunks, SQC_T, 0, s>>>(o.contrib, grad ? o.keys : nullptr, o.iters, n,
                                               max_it, L.nchunks, hist, partials, L.slots, 0, work);
   *launches = 3;
   int bwd_blocks = L.nbwd;  // rows of backward partials written
@@ -2797,7 +2820,7 @@ SqBatchLayout sq_batch_layout(const SqBatchReq* r, int K, int bwd_rows) {
   L.items = take(sizeof(SqItem) * (size_t)K);
   L.chunk_item = take(sizeof(int) * (size_t)L.chunks);
   L.claim = take(sizeof(unsigned long long));
-  L.work = take(2 * sizeof(unsigned long long));
+  L.work = take(3 * sizeof(unsigned long long));
   L.contrib = take(sizeof(double) * nf);
   L.keys = take(sizeof(int) * nf);
   L.iters = take(sizeof(int) * nf);
@@ -2868,7 +2891,7 @@ cudaError_t launch_sq_energy_batch(const SqBatchReq* r, int K, void* scratch, do
       (e = cudaMemcpyAsync(d_chunk_item, chunk_item.data(), sizeof(int) * chunk_item.size(),
                            cudaMemcpyHostToDevice, s)) ||
       (e = cudaMemsetAsync(claim, 0, sizeof(unsigned long long), s)) ||
-      (e = cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), s)))
+      (e = cudaMemsetAsync(work, 0, 3 * sizeof(unsigned long long), s)))
     return e;
   int n_launch = 0;
   sq_item_roots_kernel<<<K, 128, 0, s>>>(d_items, K);
@@ -2881,14 +2904,14 @@ cudaError_t launch_sq_energy_batch(const SqBatchReq* r, int K, void* scratch, do
   o.seed_L = reinterpret_cast<float*>(scr + L.seed_L);
   o.ck = reinterpret_cast<V4<float>*>(scr + L.ck);
   o.applied = work;
-  // persistent forward grid, as the single call's
+  // persistent forward grid, as the single request's first call
   int per_sm = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sq_fwd_batch_kernel, SQF_T, 0)))
     return e;
   const long long need = (L.n_flat + SQF_T - 1) / SQF_T;
   const int fblocks = (int)std::max<long long>(
       1, std::min<long long>((long long)sms * std::min<long long>(std::max(per_sm, 1),
-                                                                 sq_fwd_want(L.n_flat, sms)),
+                                                                 sq_fwd_want32(L.n_flat / 2, sms, per_sm)),
                             need));
   sq_fwd_batch_kernel<<<fblocks, SQF_T, 0, s>>>(d_items, d_chunk_item, L.n_flat, claim, o);
   n_launch++;
@@ -2897,7 +2920,7 @@ cudaError_t launch_sq_energy_batch(const SqBatchReq* r, int K, void* scratch, do
     const long long s0 = L.s0[(size_t)i];
     int* hist = reinterpret_cast<int*>(scr + L.hist[(size_t)i]);
     sq_chunk_kernel<<<(unsigned)L.nchunks[(size_t)i], SQC_T, 0, s>>>(
-        o.contrib + s0, o.keys + s0, r[i].n, r[i].max_it, (int)L.nchunks[(size_t)i],
+        o.contrib + s0, o.keys + s0, o.iters + s0, r[i].n, r[i].max_it, (int)L.nchunks[(size_t)i],
         hist, items[(size_t)i].partials, L.slots[(size_t)i], 0, work);
     sq_scan_kernel<<<1, 1024, 0, s>>>(hist, (long long)(r[i].max_it + 1) * L.nchunks[(size_t)i],
                                       items[(size_t)i].total);
@@ -2972,7 +2995,7 @@ cudaError_t launch_sq_energy(bool fp64, bool grad, const double* params, int nt,
                              const double* xyz, const double* target, long long n, double slice,
                              int max_it, double escape, double d_sat, void* scratch,
                              double** out, int* iters, cudaStream_t s, int* launches,
-                             unsigned long long** work) {
+                             unsigned long long** work, long long steps_hint) {
   const int sms = sm_count();
   const SqLayout L = sq_layout(fp64, grad, n, max_it, nt, nb, sms);
   unsigned char* scr = static_cast<unsigned char*>(scratch);
@@ -2980,9 +3003,9 @@ cudaError_t launch_sq_energy(bool fp64, bool grad, const double* params, int nt,
   *work = reinterpret_cast<unsigned long long*>(scr + L.work);
   if (fp64)
     return sq_launch<double>(grad, params, nt, nb, xyz, target, n, slice, max_it, escape, d_sat,
-                             scr, L, iters, sms, s, launches);
+                             scr, L, iters, sms, s, launches, steps_hint);
   return sq_launch<float>(grad, params, nt, nb, xyz, target, n, slice, max_it, escape, d_sat, scr,
-                          L, iters, sms, s, launches);
+                          L, iters, sms, s, launches, steps_hint);
 }
 
 }  // namespace qj

@@ -165,10 +165,13 @@ static int sq_energy(qjg_ctx* ctx, const double* d_params, int32_t nt, int32_t n
   double* d_out = nullptr;
   unsigned long long* d_work = nullptr;
   int launched = 0;
+  // the previous call's orbit lengths size the forward grid when it ran on as
+  // many samples with the same cap (the optimizer's repeated calls)
+  const long long hint = ctx->sq_last_n == n && ctx->sq_last_max_it == max_it ? ctx->sq_lengths : 0;
   cudaError_t e = qj::launch_sq_energy(fp64, grad, d_params, nt, nb, d_xyz, d_target, n, slice,
                                        max_it, escape, d_sat, d_scr, &d_out, d_iters, s, &launched,
-                                       &d_work);
-  unsigned long long work[2] = {0, 0};
+                                       &d_work, hint);
+  unsigned long long work[3] = {0, 0, 0};
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(work, d_work, sizeof work, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && d_grad)
@@ -180,6 +183,9 @@ static int sq_energy(qjg_ctx* ctx, const double* d_params, int32_t nt, int32_t n
   ctx->launches += launched;
   ctx->sq_applications = (int64_t)work[0];
   ctx->sq_steps = (int64_t)work[1];
+  ctx->sq_lengths = (int64_t)work[2];
+  ctx->sq_last_n = n;
+  ctx->sq_last_max_it = max_it;
   return QJG_OK;
 }
 

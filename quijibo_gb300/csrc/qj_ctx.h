@@ -51,6 +51,9 @@ struct qjg_ctx {
   int64_t launches = 0;
   int64_t sq_applications = 0;  // work of the last energy call: forward map applications
   int64_t sq_steps = 0;         // ... and adjoint orbit steps
+  int64_t sq_lengths = 0;       // its orbit lengths, sample count and iteration cap
+  int64_t sq_last_n = -1;
+  int32_t sq_last_max_it = -1;
   // marching-cubes scratch
   qj::DevStats* d_mstats = nullptr;
   double* m_field = nullptr;    // slab field window

@@ -34,14 +34,15 @@ void set_energy_adjoint_roots(int on);
 void set_energy_forward_blocks(int per_sm);
 // the FP32 polar power's fast form (hardware log2 and sin/cos, polynomial atan)
 cudaError_t set_energy_fast(int on);
-// *work: two counters in the scratch, the map applications the forward pass
-// carried out and the orbit steps of the adjoint (read after the call
-// completes).
+// *work: three counters in the scratch, the map applications the forward pass
+// carried out, the orbit steps of the adjoint and the orbit lengths (read after
+// the call completes).  steps_hint: the orbit lengths of an earlier call on as
+// many samples (0 if none), which size the FP32 forward grid and nothing else.
 cudaError_t launch_sq_energy(bool fp64, bool grad, const double* params, int nt, int nb,
                              const double* xyz, const double* target, long long n, double slice,
                              int max_it, double escape, double d_sat, void* scratch,
                              double** out, int* iters, cudaStream_t s, int* launches,
-                             unsigned long long** work);
+                             unsigned long long** work, long long steps_hint);
 
 // One request of a batch of FP32 energy + gradient calls: device pointers
 // as for launch_sq_energy.
