@@ -84,12 +84,12 @@ typedef struct {
   int64_t voxel_iters;   /* orbit lengths: map applications of the escape loop (bulk pass) */
   int64_t root_terms;    /* voxel_iters x (n_top + n_bottom) */
   int64_t refined;       /* voxels re-evaluated in FP64 */
-  int64_t refined_iters; /* map applications of the FP64 re-evaluation */
+  int64_t refined_iters; /* orbit lengths of the FP64 re-evaluation */
   int64_t nonfinite;     /* FP32 voxels that overflowed or underflowed */
   int64_t lane_iters;    /* FP32 bulk: lane slots spent (voxels of a warp x the most
                             applications one of its lanes carried out) */
   int64_t rerun;         /* voxels re-run with a double-float head (rel_tol) */
-  int64_t rerun_iters;   /* map applications of those re-runs */
+  int64_t rerun_iters;   /* orbit lengths of those re-runs */
 } qjg_field_stats;
 
 /* ---- context and root sets ------------------------------------------- */

@@ -64,9 +64,11 @@ int qjg_set_energy_adjoint_roots(int on);
 int qjg_set_energy_fast(int on);
 
 /* Process-wide block count of the energy forward kernel, for sweeps: 0 (the
- * default) the sizing rule (the resident blocks in FP32, about four samples a lane
- * in FP64, at least 3 blocks of 128 lanes per SM), else that
- * many blocks per SM, capped by residency.  With the one-sample kernel (the
+ * default) the sizing rule (in FP32 a lane for each full-length orbit of the
+ * previous call on as many samples with the same cap, half of the samples at
+ * first, or for every second, third, ... where they outnumber the resident
+ * lanes; in FP64 about four samples a lane; at least 3 blocks of 128 lanes per
+ * SM), else that many blocks per SM, capped by residency.  With the one-sample kernel (the
  * default) results do not depend on it (each sample's value is its own; sums
  * run in sample order).  Set it while no energy call is in flight; a
  * negative count returns QJG_ERR_ARG. */

@@ -644,8 +644,8 @@ __global__ void __launch_bounds__(1024) mc_scan_sums_kernel(long long* bsum2, lo
   }
 }
 
-// Pass 3: the slab's vertices and cubes in scan order.  Each thread takes
-// SCAN_V consecutive units; for the active voxels of its units it forms the
+// Pass 3: the slab's vertices and cubes in scan order.  A scan block places
+// its units; for the active voxels of each, eight lanes form the
 // edge mask and cube flag from the sign words of the voxel's unit, the unit
 // above it (y + 1), the units of the plane above, and the first column of the
 // next unit of each, and writes the vertex id base and mask of the voxel
