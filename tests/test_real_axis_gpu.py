@@ -140,3 +140,25 @@ def test_cubic(ctx, oracle, c, g):
     pair, real = z[z.imag > 1e-9][0], z[abs(z.imag) < 1e-9][0].real
     top = [[pair.real, pair.imag, 0, 0], [pair.real, -pair.imag, 0, 0], [real, 0, 0, 0]]
     _assert_polar_forms(ctx, oracle, RootSet(top_roots=np.array(top), top_powers=np.ones(3)), g)
+
+
+@pytest.mark.parametrize("form", ["polar", "integer"])
+@pytest.mark.parametrize("nt,nb", [(5, 0), (6, 3)])
+def test_mirror_images_have_the_same_bits(ctx, nt, nb, form):
+    """Roots on the real axis: the map commutes with every reflection that
+    keeps it; the cells of a 16^3 grid are each other's mirror images."""
+    rng = np.random.RandomState(nt)
+    roots = np.zeros((nt + nb, 4))
+    roots[:, 0] = rng.uniform(-1.2, 1.2, nt + nb)
+    powers = rng.uniform(0.5, 2, nt + nb) if form == "polar" else rng.choice([1.0, 2.0, 3.0], nt + nb)
+    rs = RootSet(top_roots=roots[:nt], top_powers=powers[:nt], bottom_roots=roots[nt:],
+                 bottom_powers=powers[nt:], scale=0.7)
+    g = Grid((16, 16, 16))
+    if form == "integer":
+        f = _integer_form(ctx, rs, g, 25, False).reshape(16, 16, 16)
+    else:
+        h = ctx.upload(rs)
+        f = ctx.field_host(h, g, ctx.iter_params(25, 2.0))[0]
+        ctx.free(h)
+    bits = f.view(np.uint64)
+    assert np.array_equal(bits, bits[:, ::-1]) and np.array_equal(bits, bits[::-1])
